@@ -444,9 +444,10 @@ def _run_ncc(s):
         cost, gp = ncc_value_and_grad(s["stereo"], r, src, p, s["deltas"], w, gd)
         costs.append(cost)
         grads.append(gp)
-    # the planes' three parameters have units of their own
-    return dict(cost=costs, depth=[g[..., 0] for g in grads], angles=[g[..., 1:] for g in grads],
-                trans=gd[:, :3], rot=gd[:, 3:])
+    # the planes' three parameters have units of their own; the optimiser takes f32 pose gradients
+    g = gd.to(torch.float32)
+    return dict(cost=costs, depth=[p[..., 0] for p in grads], angles=[p[..., 1:] for p in grads],
+                trans=g[:, :3], rot=g[:, 3:])
 
 
 def _work_ncc(c):
