@@ -41,6 +41,7 @@
 #include <cuda_fp16.h>
 
 #include "l3d_fmath.h"
+#include "l3d_ieee.h"
 #include "l3d_internal.h"
 
 namespace {
@@ -49,7 +50,10 @@ constexpr int TX = 16;   /* colour columns per tile */
 constexpr int TY = 8;    /* rows per tile */
 constexpr int S = 36;    /* 6 x 6 window, offsets -5, -3, ..., 5 */
 #ifndef L3D_EXACT_MIN_BLOCKS
-#define L3D_EXACT_MIN_BLOCKS 5 /* resident blocks per SM of the exact propagate kernel (5: 81 M px-iters/s on the scan, 4: 72 M) */
+/* Resident blocks per SM of the exact propagate kernel: with four the compiler has the registers to
+ * keep a row's gathers in flight, which is worth more than warps (four views of 640x480, 8 sources,
+ * 5 iterations: 4 blocks 39.2 ms, 5 47.2 ms, 6 57.5 ms). */
+#define L3D_EXACT_MIN_BLOCKS 4
 #endif
 /* Resident blocks per SM of the fast propagate kernel with the window in shared memory, with
  * gathers (4: 168.9 M px-iters/s on the scan with FP32 texels, 5: 166.8 M) and with filtered
@@ -61,11 +65,6 @@ constexpr int S = 36;    /* 6 x 6 window, offsets -5, -3, ..., 5 */
 #define L3D_SHWIN_MIN_BLOCKS 5
 #endif
 
-__device__ __forceinline__ float rcp_fast(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ float dot3f(float3 a, float3 b) {
     return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x));
 }
@@ -478,7 +477,7 @@ struct Fast {
 #pragma unroll
             for (int c = 0; c < 6; c++) {
                 const int i = r * 6 + c;
-                float iz = rcp_fast(qz);
+                float iz = l3d_rcp_approx(qz);
                 float val = GATHER ? bilinear_gather(src.tex, fmaf(qx, iz, -0.5f), fmaf(qy, iz, -0.5f))
                                    : Img<TEX>::sample(src.tex, si, src.W, src.H, qx * iz, qy * iz);
                 float sv = val - s.center;  /* s' = s - c; r' = r - c lives in rwr / rw */
@@ -500,7 +499,7 @@ struct Fast {
 #pragma unroll
                 for (int c = 0; c < 6; c++) {
                     const int i = r * 6 + c;
-                    float iz = rcp_fast(qz);
+                    float iz = l3d_rcp_approx(qz);
                     float val = pair_sample(sp, src.W, src.H, qx * iz, qy * iz);
                     float sv = val - s.center;
                     window_term(ws, s, i, sv);
@@ -615,11 +614,42 @@ struct Exact {
         s.rvar = maxw(fmaf(-s.rmean, s.rmean, srr.value() / s.rsum), 0.0f);
     }
 
+    /* The window sums of one source, every sample's position tested like the oracle does; false
+     * when one is behind the camera or outside the image.  A rolled loop: only windows that graze an
+     * image border (or leave the normal numbers) come here. */
+    __device__ bool sums_tested(const XPix& s, const L3dFastSrc& src, const float* h, Acc<COMP>& ss,
+                                Acc<COMP>& sss, Acc<COMP>& srs) const {
+        const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
+        const float2* win = exact_window();
+#pragma unroll 1
+        for (int i = 0; i < S; i++) {
+            const float x = s.px + (float)((i % 6) * 2 - 5), y = s.py + (float)((i / 6) * 2 - 5);
+            const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
+            const float qx = fmaf(h[0], x, fmaf(h[1], y, h[2]));
+            const float qy = fmaf(h[3], x, fmaf(h[4], y, h[5]));
+            const float iz = 1.0f / qz;
+            const float uu = qx * iz, vv = qy * iz;
+            if (!(qz > 1e-6f) || !(uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax)) return false;
+            const float val = bilinear_gather(src.tex, uu, vv);
+            const float2 rwv = win[i * XBLOCK];
+            ss.fma_add(rwv.x, val);
+            const float wv = rwv.x * val;
+            sss.fma_add(wv, val);
+            srs.fma_add(wv, rwv.y);
+        }
+        return true;
+    }
+
     /* view_cost (patchmatch.wgsl.ts:130-159) with H = B + kt u^T (Bt/ktt hold the unshifted
      * base in this form).  Every sample is computed as the oracle computes it; a sample with
-     * q.z <= 1e-6 or outside [0, W-1] x [0, H-1] makes the cost 2.  The four corner samples are
-     * tested first (with the same arithmetic), so most windows that leave the image stop there;
-     * the per-sample test in the loop keeps the result exact for windows that graze an edge. */
+     * q.z <= 1e-6 or outside [0, W-1] x [0, H-1] makes the cost 2.  The window's image is the convex
+     * hull of its corners' images, so four corners inside by more than the rounding of a position
+     * (`slack`, from the magnitudes that enter it: each of q's components carries three roundings,
+     * the quotient two more, and the bound allows sixteen) stand for all 36 samples: their loop is
+     * straight-line code without tests.  A window with a corner outside by as much costs 2 at once;
+     * what is left goes through sums_tested.  Bound by latency and issue: a test and a general
+     * division per sample, each a branch that cuts a row's gathers apart, took 75.6 ms for four views
+     * of 640x480 (8 sources, 5 iterations); this takes 39.2 ms. */
     __device__ float view_cost(const XPix& s, const L3dFastSrc& src, const float* u) const {
         float h[9];
 #pragma unroll
@@ -627,6 +657,7 @@ struct Exact {
 #pragma unroll
             for (int c = 0; c < 3; c++) h[r * 3 + c] = fmaf(src.ktt[r], u[c], src.Bt[r * 3 + c]);
         const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
+        float zmin = 3.0e38f, zmax = -3.0e38f, umin = 3.0e38f, umax = -3.0e38f, vmin = 3.0e38f, vmax = -3.0e38f;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             const float x = s.px + ((c & 1) ? 5.0f : -5.0f);
@@ -634,39 +665,49 @@ struct Exact {
             const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
             const float qx = fmaf(h[0], x, fmaf(h[1], y, h[2]));
             const float qy = fmaf(h[3], x, fmaf(h[4], y, h[5]));
-            const float iz = 1.0f / qz;
+            const float iz = l3d_rcp_approx(qz);
             const float uu = qx * iz, vv = qy * iz;
-            if (!(qz > 1e-6f) || !(uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax)) return 2.0f;
+            zmin = fminf(zmin, qz);
+            zmax = fmaxf(zmax, qz);
+            umin = fminf(umin, uu);
+            umax = fmaxf(umax, uu);
+            vmin = fminf(vmin, vv);
+            vmax = fmaxf(vmax, vv);
         }
+        const float ax = fabsf(s.px) + 5.0f, ay = fabsf(s.py) + 5.0f;
+        const float mz = fmaf(fabsf(h[6]), ax, fmaf(fabsf(h[7]), ay, fabsf(h[8])));
+        const float mx = fmaf(fabsf(h[0]), ax, fmaf(fabsf(h[1]), ay, fabsf(h[2])));
+        const float my = fmaf(fabsf(h[3]), ax, fmaf(fabsf(h[4]), ay, fabsf(h[5])));
+        const float unit = 0x1p-20f * l3d_rcp_approx(zmin);
+        const float su = unit * fmaf(wmax, mz, mx), sv = unit * fmaf(hmax, mz, my);
         Acc<COMP> ss, sss, srs;
-        const float2* win = exact_window();
-        bool ok = true;
+        if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv &&
+            umax <= wmax - su && vmax <= hmax - sv) {
+            const float2* win = exact_window();
 #pragma unroll
-        for (int r = 0; r < 6; r++) {
-            const float y = s.py + (float)(r * 2 - 5);
-            const float hz = fmaf(h[7], y, h[8]);
-            const float hx = fmaf(h[1], y, h[2]);
-            const float hy = fmaf(h[4], y, h[5]);
+            for (int r = 0; r < 6; r++) {
+                const float y = s.py + (float)(r * 2 - 5);
+                const float hz = fmaf(h[7], y, h[8]);
+                const float hx = fmaf(h[1], y, h[2]);
+                const float hy = fmaf(h[4], y, h[5]);
 #pragma unroll
-            for (int c = 0; c < 6; c++) {
-                const int i = r * 6 + c;
-                const float x = s.px + (float)(c * 2 - 5);
-                const float qz = fmaf(h[6], x, hz);
-                const float qx = fmaf(h[0], x, hx);
-                const float qy = fmaf(h[3], x, hy);
-                const float iz = 1.0f / qz;
-                const float uu = qx * iz, vv = qy * iz;
-                ok = ok && qz > 1e-6f && uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax;
-                const float val = bilinear_gather(src.tex, uu, vv);
-                const float2 rwv = win[i * XBLOCK];
-                const float w = rwv.x;
-                ss.fma_add(w, val);
-                const float wv = w * val;
-                sss.fma_add(wv, val);
-                srs.fma_add(wv, rwv.y);
+                for (int c = 0; c < 6; c++) {
+                    const int i = r * 6 + c;
+                    const float x = s.px + (float)(c * 2 - 5);
+                    const float iz = l3d_rcp_normal(fmaf(h[6], x, hz));
+                    const float val = bilinear_gather(src.tex, fmaf(h[0], x, hx) * iz, fmaf(h[3], x, hy) * iz);
+                    const float2 rwv = win[i * XBLOCK];
+                    const float w = rwv.x;
+                    ss.fma_add(w, val);
+                    const float wv = w * val;
+                    sss.fma_add(wv, val);
+                    srs.fma_add(wv, rwv.y);
+                }
             }
+        } else if (zmin <= 1e-6f || umin < -su || vmin < -sv || umax > wmax + su || vmax > hmax + sv ||
+                   !sums_tested(s, src, h, ss, sss, srs)) {
+            return 2.0f;
         }
-        if (!ok) return 2.0f;
         const float mean = ss.value() / s.rsum;
         const float var_s = maxw(fmaf(-mean, mean, sss.value() / s.rsum), 0.0f);
         const float den = sqrtf(s.rvar * var_s);
