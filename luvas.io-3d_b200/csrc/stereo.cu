@@ -4,8 +4,8 @@
  * Kernels of frontend/src/app/vision/mvs/patchmatch.wgsl.ts rebuilt for sm_100a: init (255-289),
  * init_coarse (296-333), propagate (349-423, one launch per colour), pack (425-433) and
  * consistency (436-469), plus a per-pixel plane-cost probe.  One thread owns one pixel; its
- * reference window (values and bilateral weights) lives in registers for the whole launch and
- * source images are read through the read-only data path (L1/L2), since each pixel's warped
+ * reference window (values and bilateral weights) lives in shared memory for the whole launch (the
+ * dense 11 x 11 window in the thread's own memory) and source images are read through the read-only data path (L1/L2), since each pixel's warped
  * footprint follows its own plane.
  *
  * Arithmetic: this form is the bit-exact twin of the FP32 CPU restatement.  The operation
@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "l3d_fmath.h"
+#include "l3d_ieee.h"
 #include "l3d_internal.h"
 
 namespace {
@@ -84,10 +85,28 @@ struct Win {
     __device__ static constexpr int oy(int i) { return (i / N) * DIL - HALF; }
 };
 
-/* Private state of one invocation (the var<private> block of patchmatch.wgsl.ts:49-54). */
+/* Private state of one invocation (the var<private> block of patchmatch.wgsl.ts:49-54).  The window's
+ * pairs (w, r) of weight and value: the 6 x 6 window's are a column of shared memory (pair i of
+ * the block's thread t at i * 128 + t, conflict-free), so that their registers go to the samples in
+ * flight; the dense 11 x 11 window's stay with the thread. */
+constexpr int kBlock = 128;
+
+template <int N>
+struct Window {
+    static constexpr bool kShared = N <= 6;
+    static constexpr int kPairs = kShared ? N * N * kBlock : 1;  /* shared pairs per block */
+    float2* column;
+    float2 own[kShared ? 1 : N * N];
+    __device__ __forceinline__ void put(int i, float2 p) {
+        if (kShared) column[i * kBlock] = p;
+        else own[i] = p;
+    }
+    __device__ __forceinline__ float2 get(int i) const { return kShared ? column[i * kBlock] : own[i]; }
+};
+
 template <int N, int DIL>
 struct Pix {
-    float rv[N * N], rw[N * N];
+    Window<N> win;
     float rsum, rmean, rvar;
     uint32_t rng;
     float px, py;
@@ -126,8 +145,7 @@ struct Stereo {
             float v = ref_pixel(x + ox, y + oy);
             float dc = v - center;
             float w = l3d_expf(-(dc * dc) / c1 - (float)(ox * ox + oy * oy) / c2);
-            s.rv[i] = v;
-            s.rw[i] = w;
+            s.win.put(i, make_float2(w, v));
             sw = sw + w;
             sr = fmaf(w, v, sr);
             srr = fmaf(w * v, v, srr);
@@ -137,22 +155,57 @@ struct Stereo {
         s.rvar = maxw(fmaf(-s.rmean, s.rmean, srr / sw), 0.0f);
     }
 
-    __device__ float bilinear(const L3dSrc& src, float u, float v) const {
-        float x0 = floorf(u), y0 = floorf(v);
-        float fx = u - x0, fy = v - y0;
-        int ix0 = (int)x0, iy0 = (int)y0;
-        int ix1 = min(ix0 + 1, src.W - 1), iy1 = min(iy0 + 1, src.H - 1);
-        const float* img = d.images + src.img_off;
-        float a = __ldg(img + (long long)iy0 * src.W + ix0);
-        float b = __ldg(img + (long long)iy0 * src.W + ix1);
-        float c = __ldg(img + (long long)iy1 * src.W + ix0);
-        float e = __ldg(img + (long long)iy1 * src.W + ix1);
-        float top = fmaf(fx, b - a, a);
-        float bot = fmaf(fx, e - c, c);
+    /* bilinear sample; INSIDE: the footprint's right and lower texels exist, so nothing is clamped */
+    template <bool INSIDE>
+    __device__ __forceinline__ float bilinear(const L3dSrc& src, float u, float v) const {
+        const float x0 = floorf(u), y0 = floorf(v);
+        const float fx = u - x0, fy = v - y0;
+        const int ix0 = (int)x0, iy0 = (int)y0;
+        const int dx = INSIDE || ix0 + 1 < src.W ? 1 : 0, dy = INSIDE || iy0 + 1 < src.H ? src.W : 0;
+        const float* t = d.images + src.img_off + (iy0 * src.W + ix0);
+        const float a = __ldg(t), b = __ldg(t + dx), c = __ldg(t + dy), e = __ldg(t + dy + dx);
+        const float top = fmaf(fx, b - a, a);
+        const float bot = fmaf(fx, e - c, c);
         return fmaf(fy, bot - top, top);
     }
 
-    /* view_cost (patchmatch.wgsl.ts:130-159) */
+    struct Sums {
+        float ss, sss, srs;
+        __device__ __forceinline__ void add(float2 p, float val) {
+            ss = fmaf(p.x, val, ss);
+            const float wv = p.x * val;
+            sss = fmaf(wv, val, sss);
+            srs = fmaf(wv, p.y, srs);
+        }
+    };
+
+    /* The window sums with every sample's position tested; false when one is behind the camera or
+     * outside the image.  A rolled loop: only windows that graze a border come here. */
+    __device__ bool sums_tested(const Pix<N, DIL>& s, const L3dSrc& src, const float* h, Sums& sum) const {
+        const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
+#pragma unroll 1
+        for (int i = 0; i < W_::S; i++) {
+            const float x = s.px + (float)W_::ox(i), y = s.py + (float)W_::oy(i);
+            const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
+            if (!(qz > 1e-6f)) return false;
+            const float qx = fmaf(h[0], x, fmaf(h[1], y, h[2]));
+            const float qy = fmaf(h[3], x, fmaf(h[4], y, h[5]));
+            const float iz = 1.0f / qz;
+            const float uu = qx * iz, vv = qy * iz;
+            if (!(uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax)) return false;
+            sum.add(s.win.get(i), bilinear<false>(src, uu, vv));
+        }
+        return true;
+    }
+
+    /* view_cost (patchmatch.wgsl.ts:130-159); a sample with q.z <= 1e-6 or outside the image makes the
+     * cost 2.  The window's image is the convex hull of its corners' images, so four corners inside
+     * by more than the rounding of a position (`slack`, from the magnitudes that enter it: each of
+     * q's components carries three roundings, the quotient two more, and the bound allows sixteen)
+     * stand for every sample, and their loop is straight-line code without tests; a corner outside
+     * by as much rejects the window at once; the rest goes through sums_tested.  One view of
+     * 640x480, 8 sources, 5 iterations: 13.4 ms; a test and a general division per sample, with the
+     * window in registers, took 38.4 ms. */
     __device__ float view_cost(const Pix<N, DIL>& s, const L3dSrc& src, const float* u) const {
         float h[9];
 #pragma unroll
@@ -160,30 +213,49 @@ struct Stereo {
 #pragma unroll
             for (int c = 0; c < 3; c++) h[r * 3 + c] = fmaf(src.kt[r], u[c], src.B[r * 3 + c]);
         const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
-        float ss = 0.0f, sss = 0.0f, srs = 0.0f;
+        constexpr float E = (float)W_::HALF;
+        float zmin = 3.0e38f, zmax = -3.0e38f, umin = 3.0e38f, umax = -3.0e38f, vmin = 3.0e38f, vmax = -3.0e38f;
 #pragma unroll
-        for (int i = 0; i < W_::S; i++) {
-            float x = s.px + (float)W_::ox(i);
-            float y = s.py + (float)W_::oy(i);
-            float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
-            if (!(qz > 1e-6f)) return 2.0f;
-            float qx = fmaf(h[0], x, fmaf(h[1], y, h[2]));
-            float qy = fmaf(h[3], x, fmaf(h[4], y, h[5]));
-            float iz = 1.0f / qz;
-            float uu = qx * iz, vv = qy * iz;
-            if (!(uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax)) return 2.0f;
-            float val = bilinear(src, uu, vv);
-            float w = s.rw[i];
-            ss = fmaf(w, val, ss);
-            float wv = w * val;
-            sss = fmaf(wv, val, sss);
-            srs = fmaf(wv, s.rv[i], srs);
+        for (int c = 0; c < 4; c++) {
+            const float x = s.px + ((c & 1) ? E : -E);
+            const float y = s.py + ((c & 2) ? E : -E);
+            const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
+            const float iz = l3d_rcp_approx(qz);
+            const float uu = fmaf(h[0], x, fmaf(h[1], y, h[2])) * iz;
+            const float vv = fmaf(h[3], x, fmaf(h[4], y, h[5])) * iz;
+            zmin = fminf(zmin, qz);
+            zmax = fmaxf(zmax, qz);
+            umin = fminf(umin, uu);
+            umax = fmaxf(umax, uu);
+            vmin = fminf(vmin, vv);
+            vmax = fmaxf(vmax, vv);
         }
-        float mean = ss / s.rsum;
-        float var_s = maxw(fmaf(-mean, mean, sss / s.rsum), 0.0f);
+        const float ax = s.px + E, ay = s.py + E;
+        const float mz = fmaf(fabsf(h[6]), ax, fmaf(fabsf(h[7]), ay, fabsf(h[8])));
+        const float mx = fmaf(fabsf(h[0]), ax, fmaf(fabsf(h[1]), ay, fabsf(h[2])));
+        const float my = fmaf(fabsf(h[3]), ax, fmaf(fabsf(h[4]), ay, fabsf(h[5])));
+        const float unit = 0x1p-20f * l3d_rcp_approx(zmin);
+        const float su = unit * fmaf(wmax, mz, mx), sv = unit * fmaf(hmax, mz, my);
+        Sums sum = {0.0f, 0.0f, 0.0f};
+        if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv &&
+            umax <= wmax - su && vmax <= hmax - sv) {
+#pragma unroll
+            for (int i = 0; i < W_::S; i++) {
+                const float x = s.px + (float)W_::ox(i), y = s.py + (float)W_::oy(i);
+                const float iz = l3d_rcp_normal(fmaf(h[6], x, fmaf(h[7], y, h[8])));
+                const float uu = fmaf(h[0], x, fmaf(h[1], y, h[2])) * iz;
+                const float vv = fmaf(h[3], x, fmaf(h[4], y, h[5])) * iz;
+                sum.add(s.win.get(i), bilinear<true>(src, uu, vv));
+            }
+        } else if (zmin <= 1e-6f || umin < -su || vmin < -sv || umax > wmax + su || vmax > hmax + sv ||
+                   !sums_tested(s, src, h, sum)) {
+            return 2.0f;
+        }
+        float mean = sum.ss / s.rsum;
+        float var_s = maxw(fmaf(-mean, mean, sum.sss / s.rsum), 0.0f);
         float den = sqrtf(s.rvar * var_s);
         if (den < 1e-5f) return 1.0f;
-        float cov = fmaf(-s.rmean, mean, srs / s.rsum);
+        float cov = fmaf(-s.rmean, mean, sum.srs / s.rsum);
         return clampw(1.0f - cov / den, 0.0f, 2.0f);
     }
 
@@ -234,7 +306,9 @@ struct Stereo {
         u[1] = (n.y * p.kinv[1]) * ir;
         u[2] = fmaf(n.x, p.kinv[2], fmaf(n.y, p.kinv[3], n.z)) * ir;
         const bool geometric = (p.flags & 1u) != 0u;
-        float costs[L3D_MAX_SOURCES];
+        /* the three smallest costs, ascending: the reference's partial selection sort adds the same
+         * values in the same order */
+        float b0 = 3.0e38f, b1 = 3.0e38f, b2 = 3.0e38f;
         for (int k = 0; k < count; k++) {
             float c = view_cost(s, p.src[k], u);
             if (geometric) {
@@ -243,20 +317,25 @@ struct Stereo {
                 float e = ok ? minw(dist, 3.0f) : 3.0f;
                 c = fmaf(p.range[3], e, c);
             }
-            costs[k] = c;
             if (view_costs) view_costs[k] = c;
+            if (c < b2) {
+                if (c < b1) {
+                    b2 = b1;
+                    if (c < b0) {
+                        b1 = b0;
+                        b0 = c;
+                    } else {
+                        b1 = c;
+                    }
+                } else {
+                    b2 = c;
+                }
+            }
         }
         const int kk = max(1, min(3, count - 1));
-        float total = 0.0f;
-        for (int pick = 0; pick < kk; pick++) {
-            int best = pick;
-            for (int j = pick + 1; j < count; j++)
-                if (costs[j] < costs[best]) best = j;
-            float tmp = costs[pick];
-            costs[pick] = costs[best];
-            costs[best] = tmp;
-            total = total + costs[pick];
-        }
+        float total = b0;
+        if (kk > 1) total = total + b1;
+        if (kk > 2) total = total + b2;
         return total / (float)kk;
     }
 
@@ -308,8 +387,10 @@ __global__ void __launch_bounds__(128) k_init(const L3dParams p, const L3dStereo
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
+    __shared__ float2 windows[Window<N>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
+    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
     st.begin(s, x, y);
     const long long index = (long long)y * p.W + x;
     float3 n = st.random_normal(s);
@@ -342,8 +423,10 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
+    __shared__ float2 windows[Window<N>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
+    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
     st.begin(s, x, y);
     const long long index = (long long)y * p.W + x;
     float3 bn = st.random_normal(s);
@@ -375,13 +458,19 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
 }
 
 /* propagate (patchmatch.wgsl.ts:349-423); threads cover the pixels of one colour. */
+/* resident blocks per SM (3: 14.2 ms for the view quoted at view_cost, 4: 13.4 ms, 5: 14.4 ms) */
+#ifndef L3D_PLAIN_MIN_BLOCKS
+#define L3D_PLAIN_MIN_BLOCKS 4
+#endif
 template <int N, int DIL>
-__global__ void __launch_bounds__(128) k_propagate(const L3dParams p, const L3dStereoDev d) {
+__global__ void __launch_bounds__(128, Window<N>::kShared ? L3D_PLAIN_MIN_BLOCKS : 1) k_propagate(const L3dParams p, const L3dStereoDev d) {
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int x = (blockIdx.x * blockDim.x + threadIdx.x) * 2 + (int)((y + p.phase) & 1u);
     if (x >= p.W || y >= p.H) return;
+    __shared__ float2 windows[Window<N>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
+    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
     st.begin(s, x, y);
     const long long index = (long long)y * p.W + x;
     float4 b = d.hyp[index];
@@ -500,8 +589,10 @@ __global__ void __launch_bounds__(128) k_plane_cost(const L3dParams p, const L3d
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
+    __shared__ float2 windows[Window<N>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
+    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
     st.begin(s, x, y);
     const long long index = (long long)y * p.W + x;
     float4 pl = planes[index];
