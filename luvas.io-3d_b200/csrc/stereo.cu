@@ -3,10 +3,10 @@
  *
  * Kernels of frontend/src/app/vision/mvs/patchmatch.wgsl.ts rebuilt for sm_100a: init (255-289),
  * init_coarse (296-333), propagate (349-423, one launch per colour), pack (425-433) and
- * consistency (436-469), plus a per-pixel plane-cost probe.  One thread owns one pixel; its
- * reference window (values and bilateral weights) lives in shared memory for the whole launch (the
- * dense 11 x 11 window in the thread's own memory) and source images are read through the read-only data path (L1/L2), since each pixel's warped
- * footprint follows its own plane.
+ * consistency (436-469), plus a per-pixel plane-cost probe.  One thread owns one
+ * pixel, eight in propagate; its reference window (values and bilateral weights) lives in shared memory for the whole launch and
+ * source images are read through the read-only data path (L1/L2), since each pixel's warped footprint
+ * follows its own plane.
  *
  * Arithmetic: this form is the bit-exact twin of the FP32 CPU restatement.  The operation
  * order is fixed (explicit fmaf, IEEE division and sqrt, l3d_fmath.h transcendentals) and the
@@ -21,6 +21,7 @@
 #include "l3d_fmath.h"
 #include "l3d_ieee.h"
 #include "l3d_internal.h"
+#include "l3d_lanes.cuh"
 
 namespace {
 
@@ -86,27 +87,28 @@ struct Win {
 };
 
 /* Private state of one invocation (the var<private> block of patchmatch.wgsl.ts:49-54).  The window's
- * pairs (w, r) of weight and value: the 6 x 6 window's are a column of shared memory (pair i of
- * the block's thread t at i * 128 + t, conflict-free), so that their registers go to the samples in
- * flight; the dense 11 x 11 window's stay with the thread. */
+ * pairs (w, r) of weight and value: the 6 x 6 window's lie in shared memory, so that their registers
+ * go to the samples in flight, pair i at column[i * STRIDE]: a column per thread of the block
+ * (STRIDE kBlock, conflict-free) or, where a pixel's lanes share a window, its pairs together
+ * (STRIDE 1, a broadcast).  The dense 11 x 11 window's stay with the thread where it is alone. */
 constexpr int kBlock = 128;
 
-template <int N>
+template <int N, int STRIDE>
 struct Window {
-    static constexpr bool kShared = N <= 6;
+    static constexpr bool kShared = N <= 6 || STRIDE == 1;
     static constexpr int kPairs = kShared ? N * N * kBlock : 1;  /* shared pairs per block */
     float2* column;
     float2 own[kShared ? 1 : N * N];
     __device__ __forceinline__ void put(int i, float2 p) {
-        if (kShared) column[i * kBlock] = p;
+        if (kShared) column[i * STRIDE] = p;
         else own[i] = p;
     }
-    __device__ __forceinline__ float2 get(int i) const { return kShared ? column[i * kBlock] : own[i]; }
+    __device__ __forceinline__ float2 get(int i) const { return kShared ? column[i * STRIDE] : own[i]; }
 };
 
-template <int N, int DIL>
+template <int N, int DIL, int STRIDE = kBlock>
 struct Pix {
-    Window<N> win;
+    Window<N, STRIDE> win;
     float rsum, rmean, rvar;
     uint32_t rng;
     float px, py;
@@ -125,7 +127,8 @@ struct Stereo {
         return make_float3((x - p.k[2]) / p.k[0], (y - p.k[3]) / p.k[1], 1.0f);
     }
 
-    __device__ float random(Pix<N, DIL>& s) const { return l3d_random(&s.rng); }
+    static __device__ __forceinline__ float dot(float3 a, float3 b) { return dot3f(a, b); }
+    static __device__ __forceinline__ float3 normalize(float3 a) { return normalize3f(a); }
 
     __device__ float ref_pixel(int x, int y) const {
         x = min(max(x, 0), p.W - 1);
@@ -133,22 +136,24 @@ struct Stereo {
         return __ldg(d.images + p.ref_off + (long long)y * p.W + x);
     }
 
-    /* prepare_window (patchmatch.wgsl.ts:90-110) */
-    __device__ void prepare_window(Pix<N, DIL>& s, int x, int y) const {
+    /* prepare_window (patchmatch.wgsl.ts:90-110): pair i of the window, and the sums in sample order */
+    __device__ float2 pair(int x, int y, int i, float center) const {
         const float c1 = 2.0f * 0.06f * 0.06f;
         const float c2 = 2.0f * 5.0f * 5.0f;
-        float center = ref_pixel(x, y);
+        const int ox = W_::ox(i), oy = W_::oy(i);
+        const float v = ref_pixel(x + ox, y + oy);
+        const float dc = v - center;
+        return make_float2(l3d_expf(-(dc * dc) / c1 - (float)(ox * ox + oy * oy) / c2), v);
+    }
+    template <class P>
+    __device__ void sums(P& s) const {
         float sw = 0.0f, sr = 0.0f, srr = 0.0f;
 #pragma unroll
         for (int i = 0; i < W_::S; i++) {
-            const int ox = W_::ox(i), oy = W_::oy(i);
-            float v = ref_pixel(x + ox, y + oy);
-            float dc = v - center;
-            float w = l3d_expf(-(dc * dc) / c1 - (float)(ox * ox + oy * oy) / c2);
-            s.win.put(i, make_float2(w, v));
-            sw = sw + w;
-            sr = fmaf(w, v, sr);
-            srr = fmaf(w * v, v, srr);
+            const float2 p = s.win.get(i);
+            sw = sw + p.x;
+            sr = fmaf(p.x, p.y, sr);
+            srr = fmaf(p.x * p.y, p.y, srr);
         }
         s.rsum = sw;
         s.rmean = sr / sw;
@@ -181,7 +186,8 @@ struct Stereo {
 
     /* The window sums with every sample's position tested; false when one is behind the camera or
      * outside the image.  A rolled loop: only windows that graze a border come here. */
-    __device__ bool sums_tested(const Pix<N, DIL>& s, const L3dSrc& src, const float* h, Sums& sum) const {
+    template <class P>
+    __device__ bool sums_tested(const P& s, const L3dSrc& src, const float* h, Sums& sum) const {
         const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
 #pragma unroll 1
         for (int i = 0; i < W_::S; i++) {
@@ -206,7 +212,8 @@ struct Stereo {
      * by as much rejects the window at once; the rest goes through sums_tested.  One view of
      * 640x480, 8 sources, 5 iterations: 13.4 ms; a test and a general division per sample, with the
      * window in registers, took 38.4 ms. */
-    __device__ float view_cost(const Pix<N, DIL>& s, const L3dSrc& src, const float* u) const {
+    template <class P>
+    __device__ float view_cost(const P& s, const L3dSrc& src, const float* u) const {
         float h[9];
 #pragma unroll
         for (int r = 0; r < 3; r++)
@@ -291,8 +298,8 @@ struct Stereo {
     }
 
     /* hypothesis_cost (patchmatch.wgsl.ts:192-233) */
-    __device__ float hypothesis_cost(const Pix<N, DIL>& s, float3 n, float dd,
-                                     float* view_costs = nullptr) const {
+    template <class P>
+    __device__ float cost_of(const P& s, float3 n, float dd, float* view_costs = nullptr) const {
         float inv = 1.0f / dd;
         if (!(dd > 0.0f) || inv > p.range[0] || inv < p.range[1]) return 2.0f;
         if (dot3f(n, s.ray) >= -1e-3f) return 2.0f;
@@ -340,9 +347,10 @@ struct Stereo {
     }
 
     /* random_normal, random_depth (patchmatch.wgsl.ts:235-249) */
-    __device__ float3 random_normal(Pix<N, DIL>& s) const {
-        float z = fmaf(random(s), 2.0f, -1.0f);
-        float a = random(s) * 6.2831853f;
+    template <class P>
+    __device__ float3 random_normal(P& s) const {
+        float z = fmaf(l3d_random(&s.rng), 2.0f, -1.0f);
+        float a = l3d_random(&s.rng) * 6.2831853f;
         float r = sqrtf(maxw(0.0f, fmaf(-z, z, 1.0f)));
         float sn, cs;
         l3d_sincosf(a, &sn, &cs);
@@ -352,46 +360,43 @@ struct Stereo {
         return normalize3f(make_float3(fmaf(view.x, -0.5f, n.x), fmaf(view.y, -0.5f, n.y),
                                        fmaf(view.z, -0.5f, n.z)));
     }
-    __device__ float random_depth(Pix<N, DIL>& s) const {
-        float t = random(s);
+    template <class P>
+    __device__ float random_depth(P& s) const {
+        float t = l3d_random(&s.rng);
         float m = fmaf(p.range[0], t, p.range[1] * (1.0f - t));
         return 1.0f / m;
     }
 
-    __device__ void begin(Pix<N, DIL>& s, int x, int y) const {
+    template <class P>
+    __device__ void begin(P& s, int x, int y) const {
         s.px = (float)x;
         s.py = (float)y;
         /* seed (patchmatch.wgsl.ts:251-253) */
         s.rng = l3d_pcg((uint32_t)(y * p.W + x) ^ l3d_pcg(p.seed + p.iter * 7919u + p.phase * 104729u));
-        prepare_window(s, x, y);
         s.ray = ray_of(s.px, s.py);
     }
-};
 
-__device__ __forceinline__ void near_offset(int i, int* ox, int* oy) {
-    int m = (i + 1) / 2;
-    *ox = (i & 1) ? -m : m;
-    *oy = -(m + 1);
-}
-__device__ __forceinline__ void orient(int ox, int oy, int dir, int* rx, int* ry) {
-    switch (dir) {
-        case 1: *rx = ox; *ry = -oy; break;
-        case 2: *rx = oy; *ry = ox; break;
-        case 3: *rx = -oy; *ry = ox; break;
-        default: *rx = ox; *ry = oy; break;
+    /* begin and the whole window by one thread */
+    template <class P>
+    __device__ void begin_window(P& s, int x, int y) const {
+        begin(s, x, y);
+        const float center = ref_pixel(x, y);
+#pragma unroll
+        for (int i = 0; i < W_::S; i++) s.win.put(i, pair(x, y, i, center));
+        sums(s);
     }
-}
+};
 
 template <int N, int DIL>
 __global__ void __launch_bounds__(128) k_init(const L3dParams p, const L3dStereoDev d) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
-    __shared__ float2 windows[Window<N>::kPairs];
+    __shared__ float2 windows[Window<N, kBlock>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
-    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
-    st.begin(s, x, y);
+    s.win.column = windows + (Window<N, kBlock>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
+    st.begin_window(s, x, y);
     const long long index = (long long)y * p.W + x;
     float3 n = st.random_normal(s);
     float dd = st.random_depth(s);
@@ -402,12 +407,12 @@ __global__ void __launch_bounds__(128) k_init(const L3dParams p, const L3dStereo
             n = unpack_normal(packed);
         }
     }
-    float c = st.hypothesis_cost(s, n, dd);
+    float c = st.cost_of(s, n, dd);
     if (!(p.flags & 1u) && d.prior && d.prior[index] > 0.0f) {
         float3 v = normalize3f(s.ray);
         float3 pn = make_float3(-v.x, -v.y, -v.z);
         float pd = d.prior[index];
-        float pc = st.hypothesis_cost(s, pn, pd);
+        float pc = st.cost_of(s, pn, pd);
         if (pc < c) {
             c = pc;
             n = pn;
@@ -423,15 +428,15 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
-    __shared__ float2 windows[Window<N>::kPairs];
+    __shared__ float2 windows[Window<N, kBlock>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
-    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
-    st.begin(s, x, y);
+    s.win.column = windows + (Window<N, kBlock>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
+    st.begin_window(s, x, y);
     const long long index = (long long)y * p.W + x;
     float3 bn = st.random_normal(s);
     float bd = st.random_depth(s);
-    float best_cost = st.hypothesis_cost(s, bn, bd);
+    float best_cost = st.cost_of(s, bn, bd);
     float qx = ((s.px + 0.5f) * (float)p.cW) / (float)p.W - 0.5f;
     float qy = ((s.py + 0.5f) * (float)p.cH) / (float)p.H - 0.5f;
     int bx = (int)floorf(qx), by = (int)floorf(qy);
@@ -446,7 +451,7 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
         float den = dot3f(hn, s.ray);
         if (fabsf(den) < 1e-6f) continue;
         float dd = dot3f(hn, point) / den;
-        float c = st.hypothesis_cost(s, hn, dd);
+        float c = st.cost_of(s, hn, dd);
         if (c < best_cost) {
             best_cost = c;
             bn = hn;
@@ -457,86 +462,33 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
     d.cost[index] = best_cost;
 }
 
-/* propagate (patchmatch.wgsl.ts:349-423); threads cover the pixels of one colour. */
-/* resident blocks per SM (3: 14.2 ms for the view quoted at view_cost, 4: 13.4 ms, 5: 14.4 ms) */
-#ifndef L3D_PLAIN_MIN_BLOCKS
-#define L3D_PLAIN_MIN_BLOCKS 4
-#endif
+/* propagate (patchmatch.wgsl.ts:349-423), eight lanes per pixel (l3d_lanes.cuh): a warp holds a 2 x 2
+ * block of the colour's pixels, a block 8 x 2.  Bound by issue and the latency of the sample loads, so
+ * resident warps pay more than registers: seven blocks per SM (the 6 x 6 window at 640x480, 8
+ * sources, 3 iterations: 4 blocks 9.1 ms, 5 8.3, 7 8.15, 8 8.2, 10 9.3).  A thread per pixel with the
+ * window in a shared-memory column took 8.4 ms there, 38.8 against 36.2 ms at 1280x960 and 1.6
+ * against 0.61 ms at 160x120, so no size keeps it.  The dense 11 x 11 window, whose pairs a thread alone
+ * keeps in local memory, went from 53.7 to 13.0 ms at 640x480 (4 sources, 2 iterations). */
+constexpr int kPropagateBlocks = 7;
 template <int N, int DIL>
-__global__ void __launch_bounds__(128, Window<N>::kShared ? L3D_PLAIN_MIN_BLOCKS : 1) k_propagate(const L3dParams p, const L3dStereoDev d) {
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    const int x = (blockIdx.x * blockDim.x + threadIdx.x) * 2 + (int)((y + p.phase) & 1u);
-    if (x >= p.W || y >= p.H) return;
-    __shared__ float2 windows[Window<N>::kPairs];
+__global__ void __launch_bounds__(128, kPropagateBlocks) k_propagate(const L3dParams p, const L3dStereoDev d) {
+    __shared__ float2 windows[N * N * 16];
+    const int warp = threadIdx.x >> 5, sub = (threadIdx.x >> 3) & 3, cand = threadIdx.x & 7;
+    int y = blockIdx.y * 2 + (sub >> 1);
+    int x = (blockIdx.x * 8 + warp * 2 + (sub & 1)) * 2 + (int)((y + p.phase) & 1u);
+    const bool inside = x < p.W && y < p.H;
+    if (!__any_sync(0xffffffffu, inside)) return;
+    x = min(x, p.W - 1);  /* lanes outside the image stay for the shuffles and write nothing */
+    y = min(y, p.H - 1);
     Stereo<N, DIL> st(p, d);
-    Pix<N, DIL> s;
-    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
+    Pix<N, DIL, 1> s;
+    s.win.column = windows + (warp * 4 + sub) * (N * N);
     st.begin(s, x, y);
-    const long long index = (long long)y * p.W + x;
-    float4 b = d.hyp[index];
-    float3 bn = make_float3(b.x, b.y, b.z);
-    float bd = b.w;
-    float best_cost = d.cost[index];
-    for (int region = 0; region < 8; region++) {
-        const int count = region < 4 ? 7 : 11;
-        long long chosen = -1;
-        float chosen_cost = 1e9f;
-        for (int i = 0; i < count; i++) {
-            int ox = 0, oy = -3 - 2 * i;
-            if (region < 4) near_offset(i, &ox, &oy);
-            int rx, ry;
-            orient(ox, oy, region & 3, &rx, &ry);
-            int qx = x + rx, qy = y + ry;
-            if (qx < 0 || qy < 0 || qx >= p.W || qy >= p.H) continue;
-            long long qi = (long long)qy * p.W + qx;
-            float c = d.cost[qi];
-            if (c < chosen_cost) {
-                chosen_cost = c;
-                chosen = qi;
-            }
-        }
-        if (chosen < 0) continue;
-        float4 h = d.hyp[chosen];
-        float3 hn = make_float3(h.x, h.y, h.z);
-        float3 rq = st.ray_of((float)(chosen % p.W), (float)(chosen / p.W));
-        float den = dot3f(hn, s.ray);
-        if (fabsf(den) < 1e-6f) continue;
-        float dd = dot3f(hn, make_float3(rq.x * h.w, rq.y * h.w, rq.z * h.w)) / den;
-        float c = st.hypothesis_cost(s, hn, dd);
-        if (c < best_cost) {
-            best_cost = c;
-            bn = hn;
-            bd = dd;
-        }
-    }
-    const float step = p.range[2];
-    float3 view = normalize3f(s.ray);
-    float3 n_random = st.random_normal(s);
-    float d_random = st.random_depth(s);
-    float e = (fmaf(st.random(s), 2.0f, -1.0f) * 0.15f) * step;
-    float d_perturbed = 1.0f / ((1.0f / bd) * (1.0f + e));
-    float r1 = st.random(s), r2 = st.random(s), r3 = st.random(s);
-    float3 np = make_float3(bn.x + (fmaf(r1, 2.0f, -1.0f) * 0.6f) * step,
-                            bn.y + (fmaf(r2, 2.0f, -1.0f) * 0.6f) * step,
-                            bn.z + (fmaf(r3, 2.0f, -1.0f) * 0.6f) * step);
-    float3 n_perturbed = normalize3f(np);
-    if (dot3f(n_perturbed, view) >= 0.0f) n_perturbed = bn;
-    const float3 cur_n = bn;
-    const float cur_d = bd;
-    for (int c = 0; c < 6; c++) {
-        /* candidates (n_random, d_random), (n_perturbed, d_perturbed), (current, d_random),
-         * (n_random, current), (current, d_perturbed), (n_perturbed, current) */
-        float3 nn = (c == 0 || c == 3) ? n_random : ((c == 1 || c == 5) ? n_perturbed : cur_n);
-        float dv = (c == 0 || c == 2) ? d_random : ((c == 1 || c == 4) ? d_perturbed : cur_d);
-        float cand = st.hypothesis_cost(s, nn, dv);
-        if (cand < best_cost) {
-            best_cost = cand;
-            bn = nn;
-            bd = dv;
-        }
-    }
-    d.hyp[index] = make_float4(bn.x, bn.y, bn.z, bd);
-    d.cost[index] = best_cost;
+    const float center = st.ref_pixel(x, y);
+    for (int i = cand; i < N * N; i += 8) s.win.put(i, st.pair(x, y, i, center));
+    __syncwarp();
+    st.sums(s);
+    l3d_step_lanes(st, s, d.hyp, d.cost, x, y, p.W, p.H, inside, cand, p.range[2]);
 }
 
 __global__ void k_pack(const L3dParams p, const L3dStereoDev d) {
@@ -589,16 +541,16 @@ __global__ void __launch_bounds__(128) k_plane_cost(const L3dParams p, const L3d
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= p.W || y >= p.H) return;
-    __shared__ float2 windows[Window<N>::kPairs];
+    __shared__ float2 windows[Window<N, kBlock>::kPairs];
     Stereo<N, DIL> st(p, d);
     Pix<N, DIL> s;
-    s.win.column = windows + (Window<N>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
-    st.begin(s, x, y);
+    s.win.column = windows + (Window<N, kBlock>::kShared ? threadIdx.y * blockDim.x + threadIdx.x : 0);
+    st.begin_window(s, x, y);
     const long long index = (long long)y * p.W + x;
     float4 pl = planes[index];
     float vc[L3D_MAX_SOURCES];
     for (int k = 0; k < L3D_MAX_SOURCES; k++) vc[k] = 0.0f;
-    cost[index] = st.hypothesis_cost(s, make_float3(pl.x, pl.y, pl.z), pl.w, vc);
+    cost[index] = st.cost_of(s, make_float3(pl.x, pl.y, pl.z), pl.w, vc);
     if (view_costs)
         for (int k = 0; k < L3D_MAX_SOURCES; k++) view_costs[index * L3D_MAX_SOURCES + k] = vc[k];
 }
@@ -618,9 +570,8 @@ cudaError_t launch_win(int kernel, const L3dParams& p, const L3dStereoDev& d, cu
             break;
         }
         case L3D_K_PROPAGATE: {
-            int half = (p.W + 1) / 2;
-            dim3 grid((half + 31) / 32, (p.H + 3) / 4);
-            k_propagate<N, DIL><<<grid, block, 0, stream>>>(p, d);
+            const int half = (p.W + 1) / 2;
+            k_propagate<N, DIL><<<dim3((half + 7) / 8, (p.H + 1) / 2), 128, 0, stream>>>(p, d);
             break;
         }
         default:
