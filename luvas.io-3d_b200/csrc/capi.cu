@@ -1383,13 +1383,7 @@ int l3d_stereo_autotune(l3d_stereo* s, int32_t n_refs, const int32_t* refs,
     }
     const bool six_only = s->opts.form == L3D_FORM_EXACT || s->opts.compensated || !s->pairs ||
                           (s->variant & 16);
-    /* +32 (the window in shared memory) is a fast-form option; BF16 returned above */
-    const bool shwin = s->opts.form == L3D_FORM_FAST;
-    std::vector<int> candidates = six_only ? std::vector<int>{6, 14} : std::vector<int>{6, 14, 4, 12};
-    if (shwin) {
-        candidates.push_back(6 | 32);
-        candidates.push_back(14 | 32);
-    }
+    std::vector<int> candidates = six_only ? std::vector<int>{14} : std::vector<int>{14, 12};
     /* up to three iterations: the first propagates random planes, the later ones the converging
      * planes whose neighbouring pixels agree, and the variants rank differently on the two */
     std::vector<l3d_solve_opts> one(opts, opts + n_refs);

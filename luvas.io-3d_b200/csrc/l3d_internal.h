@@ -165,8 +165,8 @@ struct L3dFastDev {
 
 /* kernel: L3D_K_INIT or L3D_K_PROPAGATE; iteration/phase select the RNG stream and the
  * refinement step; views with fewer iterations than `iteration + 1` are skipped.  variant:
- * window rows sampled by the texture unit (0..6, the rest from the pair image) + 8 for the 2x2
- * quad lane mapping. */
+ * window rows sampled by the texture unit (6, 4, 3 or 2, the rest from the pair image) + 16 for
+ * gathers with exact weights. */
 cudaError_t l3d_launch_fast(int kernel, const L3dFastDev& d, int iteration, int phase,
                             int variant, cudaStream_t stream);
 /* pair image of one layer: half2(texel, right neighbour) from the linear storage */

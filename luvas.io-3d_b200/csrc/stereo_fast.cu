@@ -36,34 +36,36 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <type_traits>
-
 #include <cuda_fp16.h>
 
 #include "l3d_fmath.h"
 #include "l3d_ieee.h"
 #include "l3d_internal.h"
+#include "l3d_lanes.cuh"
 
 namespace {
 
 constexpr int TX = 16;   /* colour columns per tile */
 constexpr int TY = 8;    /* rows per tile */
 constexpr int S = 36;    /* 6 x 6 window, offsets -5, -3, ..., 5 */
-#ifndef L3D_EXACT_MIN_BLOCKS
-/* Resident blocks per SM of the exact propagate kernel: with four the compiler has the registers to
- * keep a row's gathers in flight, which is worth more than warps (four views of 640x480, 8 sources,
- * 5 iterations: 4 blocks 39.2 ms, 5 47.2 ms, 6 57.5 ms). */
-#define L3D_EXACT_MIN_BLOCKS 4
-#endif
-/* Resident blocks per SM of the fast propagate kernel with the window in shared memory, with
- * gathers (4: 168.9 M px-iters/s on the scan with FP32 texels, 5: 166.8 M) and with filtered
- * samples (5: 249.7 M with FP16 texels, 4: 248.0 M). */
-#ifndef L3D_SHWIN_GATHER_MIN_BLOCKS
-#define L3D_SHWIN_GATHER_MIN_BLOCKS 4
-#endif
-#ifndef L3D_SHWIN_MIN_BLOCKS
-#define L3D_SHWIN_MIN_BLOCKS 5
-#endif
+/* How the propagate step is laid out for one evaluator: resident blocks per SM of the kernel with a
+ * thread per pixel and of the one with eight lanes per pixel (l3d_lanes.cuh), and the largest launch,
+ * in 128-pixel tiles of one colour, that takes the lanes. */
+struct Layout {
+    int blocks, lane_blocks, lane_tiles;
+};
+/* Measured at 640x480, 8 sources, 3 iterations (ms, thread / lanes), 300, 675, 1200, 2400, 4800
+ * tiles.  Filtered samples keep the texture pipe busy either way; the lanes win while the thread
+ * kernel's last wave is a large part of it: 1.25 / 0.97, 2.36 / 2.04, 3.99 / 3.69, 7.69 / 7.57,
+ * 15.7 / 15.8. */
+constexpr Layout kFilter = {5, 5, 3000};
+/* Gathers are bound by latency and issue; a quarter of the lanes idle in the lanes' second round:
+ * 1.81 / 1.54, 4.00 / 3.24, 5.68 / 5.75. */
+constexpr Layout kGather = {4, 5, 1000};
+/* The exact evaluator likewise: 2.13 / 1.72, 4.41 / 3.77, 6.47 / 6.81.  With four blocks the compiler
+ * has the registers to keep a row's gathers in flight, which is worth more than warps (four views,
+ * 5 iterations, thread per pixel: 4 blocks 39.2 ms, 5 47.2 ms, 6 57.5 ms). */
+constexpr Layout kExact = {4, 4, 1000};
 
 __device__ __forceinline__ float dot3f(float3 a, float3 b) {
     return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x));
@@ -106,6 +108,17 @@ struct Acc {
         else s = fmaf(a, b, s);
     }
     __device__ __forceinline__ float value() const { return COMP ? s + c : s; }
+};
+
+/* The three sums over a reference window's pairs (w, a): sum w, sum w a, sum w a^2. */
+template <bool COMP>
+struct RefSums {
+    Acc<COMP> sw, sr, srr;
+    __device__ __forceinline__ void add(float2 p) {
+        sw.add(p.x);
+        sr.fma_add(p.x, p.y);
+        srr.fma_add(p.x * p.y, p.y);
+    }
 };
 
 /* The three source-window sums of the fast evaluator (sum w s', sum w s'^2, sum w r' s' over
@@ -297,9 +310,9 @@ __device__ __forceinline__ bool reproject(const L3dFastView& v, const L3dFastDev
  * orientation tests, u = (K_r^-T n) / rho, per-source cost (+ geometric term), mean of the
  * k = max(1, min(3, S - 1)) smallest.  The three smallest are kept in registers, ascending; the
  * reference's partial selection sort adds the same values in the same order. */
-template <class E>
+template <class E, class P>
 __device__ __forceinline__ float hyp_cost(const E& e, const L3dFastView& v, const L3dFastDev& d,
-                                          const typename E::Pix& s, float3 n, float dd) {
+                                          const P& s, float3 n, float dd) {
     if (!(dd > 0.0f)) return 2.0f;
     float inv = 1.0f / dd;
     if (inv > v.range[0] || inv < v.range[1]) return 2.0f;
@@ -342,48 +355,62 @@ __device__ __forceinline__ float hyp_cost(const E& e, const L3dFastView& v, cons
     return total / (float)kk;
 }
 
-/* This thread's window column in shared memory: element i (sample i's pair of window values)
- * at [i * XBLOCK]; consecutive threads read consecutive float2, so a warp's access is
- * conflict-free.  The exact evaluator keeps (w, r) there, the fast evaluator with a shared
- * window (w, w (r - c)). */
+/* One pixel's reference window in shared memory: 36 pairs of window values, pair i at
+ * win[i * STRIDE].  The propagate kernel keeps a pixel's pairs together (STRIDE 1: the eight lanes
+ * of a pixel read the same pair, a broadcast); the kernels with one thread per pixel keep a column
+ * per thread (STRIDE 128: consecutive threads read consecutive pairs).  The exact evaluator's pairs
+ * are (w, r), the fast evaluator's (w, w (r - c)), c the centre pixel. */
 constexpr int XBLOCK = 128;
-__device__ __forceinline__ float2* exact_window() {
-    __shared__ float2 win[S * XBLOCK];
-    return win + threadIdx.x;
-}
 
-/* Per-pixel state: the reference window as w and w (r - c), c = centre pixel. */
+/* Per-pixel state of the fast evaluator. */
+template <int STRIDE>
 struct FPix {
-    float rw[S], rwr[S];
+    static constexpr int kStride = STRIDE;
+    const float2* win;
     float center, inv_sum, mean_r, var_r;
     uint32_t rng;
     float px, py;
     float3 ray;
 };
 
-/* The same without the window, which lives in shared memory (exact_window). */
-struct FPixS {
-    float center, inv_sum, mean_r, var_r;
-    uint32_t rng;
-    float px, py;
-    float3 ray;
+/* What the evaluators share: the view and the buffers, rays and random depths. */
+struct Scene {
+    const L3dFastView& v;
+    const L3dFastDev& d;
+    __device__ Scene(const L3dFastView& view, const L3dFastDev& dev) : v(view), d(dev) {}
+
+    static __device__ __forceinline__ float dot(float3 a, float3 b) { return dot3f(a, b); }
+    __device__ float3 ray_of(float x, float y) const {
+        return make_float3((x - v.k[2]) / v.k[0], (y - v.k[3]) / v.k[1], 1.0f);
+    }
+    /* random_depth (patchmatch.wgsl.ts:243-249) */
+    template <class P>
+    __device__ float random_depth(P& s) const {
+        float t = l3d_random(&s.rng);
+        return 1.0f / fmaf(v.range[0], t, v.range[1] * (1.0f - t));
+    }
+    /* The pixel's RNG state, coordinates and ray (seed, patchmatch.wgsl.ts:251-253). */
+    template <class P>
+    __device__ void begin(P& s, int x, int y, int iteration, int phase) const {
+        s.px = (float)x;
+        s.py = (float)y;
+        uint32_t seed = (uint32_t)(v.ref + 1) * 0x9e3779b1u + (uint32_t)iteration * 97u +
+                        (uint32_t)phase * 13u + (v.flags & 1u) * 7u;
+        s.rng = l3d_pcg((uint32_t)(y * v.W + x) ^
+                        l3d_pcg(seed + (uint32_t)iteration * 7919u + (uint32_t)phase * 104729u));
+        s.ray = ray_of(s.px, s.py);
+    }
 };
 
 /* TEX: texture-unit sampling of F16/F32 arrays (false: BF16 linear memory).  TEXROWS: window
  * rows (of 6) sampled by the texture unit; the other rows use pair_sample (TEX only).  COMP:
  * compensated window sums.  GATHER: the texture rows are texture gathers weighted with exact
- * FP32 bilinear weights instead of hardware-filtered fetches (8-bit weights).  SHWIN: the
- * reference window lives in shared memory instead of 72 registers, so that more warps are
- * resident to cover the texture latency; the arithmetic, and so every result, is unchanged. */
-template <bool TEX, int TEXROWS = 6, bool COMP = false, bool GATHER = false, bool SHWIN = false>
-struct Fast {
-    using Pix = typename std::conditional<SHWIN, FPixS, FPix>::type;
-    /* resident blocks per SM the propagate kernel targets */
-    static constexpr int kMinBlocks =
-        SHWIN ? (GATHER ? L3D_SHWIN_GATHER_MIN_BLOCKS : L3D_SHWIN_MIN_BLOCKS) : 3;
-    const L3dFastView& v;
-    const L3dFastDev& d;
-    __device__ Fast(const L3dFastView& view, const L3dFastDev& dev) : v(view), d(dev) {}
+ * FP32 bilinear weights instead of hardware-filtered fetches (8-bit weights). */
+template <bool TEX, int TEXROWS = 6, bool COMP = false, bool GATHER = false>
+struct Fast : Scene {
+    template <int STRIDE> using Pix = FPix<STRIDE>;
+    static constexpr Layout kLayout = GATHER ? kGather : kFilter;
+    using Scene::Scene;
 
     static __device__ __forceinline__ float3 normalize(float3 a) { return normalize_fast(a); }
     static __device__ __forceinline__ float3 unpack_n(uint32_t packed) { return unpack_normal(packed); }
@@ -392,53 +419,40 @@ struct Fast {
         return (const uint16_t*)d.images + off;
     }
 
-    __device__ float3 ray_of(float x, float y) const {
-        return make_float3((x - v.k[2]) / v.k[0], (y - v.k[3]) / v.k[1], 1.0f);
+    /* prepare_window (patchmatch.wgsl.ts:90-110), shifted by the centre pixel, in three steps so
+     * that the lanes of a pixel can share the first: the centre, pair i as (w, r - c), and the
+     * sums in sample order; scale() turns a pair into the stored (w, w (r - c)). */
+    __device__ float center(int x, int y) const {
+        return Img<TEX>::texel(v.ref_tex, img(v.ref_img_off), v.W, v.H, x, y);
     }
-
-    __device__ float random(Pix& s) const { return l3d_random(&s.rng); }
-
-    /* prepare_window (patchmatch.wgsl.ts:90-110), shifted by the centre pixel */
-    __device__ void prepare(Pix& s, int x, int y) const {
-        const uint16_t* ri = img(v.ref_img_off);
-        const float center = Img<TEX>::texel(v.ref_tex, ri, v.W, v.H, x, y);
+    __device__ float2 pair(int x, int y, int i, float c) const {
         const float ic1 = 1.0f / (2.0f * 0.06f * 0.06f);
-        Acc<COMP> sw, sr, srr;
-#pragma unroll
-        for (int i = 0; i < S; i++) {
-            const int ox = (i % 6) * 2 - 5, oy = (i / 6) * 2 - 5;
-            const float spatial = (float)(ox * ox + oy * oy) / (2.0f * 5.0f * 5.0f);
-            float val = Img<TEX>::texel(v.ref_tex, ri, v.W, v.H, x + ox, y + oy);
-            float dc = val - center;
-            float w = __expf(-(dc * dc) * ic1 - spatial);
-            if constexpr (SHWIN) {
-                exact_window()[i * XBLOCK] = make_float2(w, w * dc);
-            } else {
-                s.rw[i] = w;
-                s.rwr[i] = w * dc;
-            }
-            sw.add(w);
-            sr.fma_add(w, dc);
-            srr.fma_add(w * dc, dc);
-        }
-        s.center = center;
-        s.inv_sum = 1.0f / sw.value();
-        s.mean_r = sr.value() * s.inv_sum;
-        s.var_r = fmaxf(fmaf(-s.mean_r, s.mean_r, srr.value() * s.inv_sum), 0.0f);
+        const int ox = (i % 6) * 2 - 5, oy = (i / 6) * 2 - 5;
+        const float spatial = (float)(ox * ox + oy * oy) / (2.0f * 5.0f * 5.0f);
+        const float val = Img<TEX>::texel(v.ref_tex, img(v.ref_img_off), v.W, v.H, x + ox, y + oy);
+        const float dc = val - c;
+        return make_float2(__expf(-(dc * dc) * ic1 - spatial), dc);
     }
+    using Sums = RefSums<COMP>;
+    template <class P>
+    __device__ void finish(P& s, const Sums& m, float c) const {
+        s.center = c;
+        s.inv_sum = 1.0f / m.sw.value();
+        s.mean_r = m.sr.value() * s.inv_sum;
+        s.var_r = fmaxf(fmaf(-s.mean_r, s.mean_r, m.srr.value() * s.inv_sum), 0.0f);
+    }
+    static __device__ __forceinline__ float2 scale(float2 p) { return make_float2(p.x, p.x * p.y); }
 
     /* one sample's terms of the window sums: w s', s' and (w r') s' (s' = s - c, r' = r - c) */
-    static __device__ __forceinline__ void window_term(WinSums<COMP>& ws, const Pix& s, int i, float sv) {
-        if constexpr (SHWIN) {
-            const float2 w = exact_window()[i * XBLOCK];
-            ws.term(w.x * sv, sv, w.y);
-        } else {
-            ws.term(s.rw[i] * sv, sv, s.rwr[i]);
-        }
+    template <class P>
+    static __device__ __forceinline__ void window_term(WinSums<COMP>& ws, const P& s, int i, float sv) {
+        const float2 w = s.win[i * P::kStride];
+        ws.term(w.x * sv, sv, w.y);
     }
 
     /* view_cost (patchmatch.wgsl.ts:130-159) with H = Bt + ktt u^T. */
-    __device__ float view_cost(const Pix& s, const L3dFastSrc& src, const float* u) const {
+    template <class P>
+    __device__ float view_cost(const P& s, const L3dFastSrc& src, const float* u) const {
         float h[9];
 #pragma unroll
         for (int r = 0; r < 3; r++)
@@ -480,7 +494,7 @@ struct Fast {
                 float iz = l3d_rcp_approx(qz);
                 float val = GATHER ? bilinear_gather(src.tex, fmaf(qx, iz, -0.5f), fmaf(qy, iz, -0.5f))
                                    : Img<TEX>::sample(src.tex, si, src.W, src.H, qx * iz, qy * iz);
-                float sv = val - s.center;  /* s' = s - c; r' = r - c lives in rwr / rw */
+                float sv = val - s.center;
                 window_term(ws, s, i, sv);
                 qx += dxx;
                 qy += dxy;
@@ -522,14 +536,16 @@ struct Fast {
     }
 
     /* hypothesis_cost (patchmatch.wgsl.ts:192-233) */
-    __device__ float hypothesis_cost(const Pix& s, float3 n, float dd) const {
+    template <class P>
+    __device__ float cost_of(const P& s, float3 n, float dd) const {
         return hyp_cost(*this, v, d, s, n, dd);
     }
 
-    /* random_normal, random_depth (patchmatch.wgsl.ts:235-249) */
-    __device__ float3 random_normal(Pix& s) const {
-        float z = fmaf(random(s), 2.0f, -1.0f);
-        float a = random(s) * 6.2831853f;
+    /* random_normal (patchmatch.wgsl.ts:235-242) */
+    template <class P>
+    __device__ float3 random_normal(P& s) const {
+        float z = fmaf(l3d_random(&s.rng), 2.0f, -1.0f);
+        float a = l3d_random(&s.rng) * 6.2831853f;
         float r = sqrtf(fmaxf(0.0f, fmaf(-z, z, 1.0f)));
         float sn, cs;
         __sincosf(a, &sn, &cs);
@@ -539,28 +555,13 @@ struct Fast {
         return normalize_fast(make_float3(fmaf(view.x, -0.5f, n.x), fmaf(view.y, -0.5f, n.y),
                                           fmaf(view.z, -0.5f, n.z)));
     }
-    __device__ float random_depth(Pix& s) const {
-        float t = random(s);
-        return 1.0f / fmaf(v.range[0], t, v.range[1] * (1.0f - t));
-    }
-
-    __device__ void begin(Pix& s, int x, int y, int iteration, int phase) const {
-        s.px = (float)x;
-        s.py = (float)y;
-        uint32_t seed = (uint32_t)(v.ref + 1) * 0x9e3779b1u + (uint32_t)iteration * 97u +
-                        (uint32_t)phase * 13u + (v.flags & 1u) * 7u;
-        s.rng = l3d_pcg((uint32_t)(y * v.W + x) ^
-                        l3d_pcg(seed + (uint32_t)iteration * 7919u + (uint32_t)phase * 104729u));
-        prepare(s, x, y);
-        s.ray = ray_of(s.px, s.py);
-    }
 };
 
-/* Per-pixel state of the exact evaluator: the private block of patchmatch.wgsl.ts:49-54.  The
- * window's bilateral weights and values (w, v) live in shared memory, one column of S float2 per
- * thread (exact_window), so that the registers they would take go to more resident warps and
- * more gathers in flight; the weighted sum, mean and variance stay in registers. */
+/* Per-pixel state of the exact evaluator: the private block of patchmatch.wgsl.ts:49-54. */
+template <int STRIDE>
 struct XPix {
+    static constexpr int kStride = STRIDE;
+    const float2* win;
     float rsum, rmean, rvar;
     uint32_t rng;
     float px, py;
@@ -570,21 +571,13 @@ struct XPix {
 /* The plain form's arithmetic in the batched kernels (see the file header).  COMP: Neumaier-
  * compensated window sums (the oracle's compensated mode). */
 template <bool COMP>
-struct Exact {
-    using Pix = XPix;
-    static constexpr int kMinBlocks = L3D_EXACT_MIN_BLOCKS;
-    const L3dFastView& v;
-    const L3dFastDev& d;
-    __device__ Exact(const L3dFastView& view, const L3dFastDev& dev) : v(view), d(dev) {}
+struct Exact : Scene {
+    template <int STRIDE> using Pix = XPix<STRIDE>;
+    static constexpr Layout kLayout = kExact;
+    using Scene::Scene;
 
     static __device__ __forceinline__ float3 normalize(float3 a) { return normalize_ieee(a); }
     static __device__ __forceinline__ float3 unpack_n(uint32_t packed) { return unpack_normal_ieee(packed); }
-
-    __device__ float3 ray_of(float x, float y) const {
-        return make_float3((x - v.k[2]) / v.k[0], (y - v.k[3]) / v.k[1], 1.0f);
-    }
-
-    __device__ float random(XPix& s) const { return l3d_random(&s.rng); }
 
     __device__ float ref_pixel(int x, int y) const {
         x = min(max(x, 0), v.W - 1);
@@ -592,35 +585,32 @@ struct Exact {
         return __ldg((const float*)d.images + v.ref_img_off + (long long)y * v.W + x);
     }
 
-    /* prepare_window (patchmatch.wgsl.ts:90-110) */
-    __device__ void prepare(XPix& s, int x, int y) const {
+    /* prepare_window (patchmatch.wgsl.ts:90-110), split like the fast evaluator's */
+    __device__ float center(int x, int y) const { return ref_pixel(x, y); }
+    __device__ float2 pair(int x, int y, int i, float c) const {
         const float c1 = 2.0f * 0.06f * 0.06f;
         const float c2 = 2.0f * 5.0f * 5.0f;
-        const float center = ref_pixel(x, y);
-        Acc<COMP> sw, sr, srr;
-#pragma unroll
-        for (int i = 0; i < S; i++) {
-            const int ox = (i % 6) * 2 - 5, oy = (i / 6) * 2 - 5;
-            float val = ref_pixel(x + ox, y + oy);
-            float dc = val - center;
-            float w = l3d_expf(-(dc * dc) / c1 - (float)(ox * ox + oy * oy) / c2);
-            exact_window()[i * XBLOCK] = make_float2(w, val);
-            sw.add(w);
-            sr.fma_add(w, val);
-            srr.fma_add(w * val, val);
-        }
-        s.rsum = sw.value();
-        s.rmean = sr.value() / s.rsum;
-        s.rvar = maxw(fmaf(-s.rmean, s.rmean, srr.value() / s.rsum), 0.0f);
+        const int ox = (i % 6) * 2 - 5, oy = (i / 6) * 2 - 5;
+        const float val = ref_pixel(x + ox, y + oy);
+        const float dc = val - c;
+        return make_float2(l3d_expf(-(dc * dc) / c1 - (float)(ox * ox + oy * oy) / c2), val);
     }
+    using Sums = RefSums<COMP>;
+    template <class P>
+    __device__ void finish(P& s, const Sums& m, float) const {
+        s.rsum = m.sw.value();
+        s.rmean = m.sr.value() / s.rsum;
+        s.rvar = maxw(fmaf(-s.rmean, s.rmean, m.srr.value() / s.rsum), 0.0f);
+    }
+    static __device__ __forceinline__ float2 scale(float2 p) { return p; }
 
     /* The window sums of one source, every sample's position tested like the oracle does; false
      * when one is behind the camera or outside the image.  A rolled loop: only windows that graze an
      * image border (or leave the normal numbers) come here. */
-    __device__ bool sums_tested(const XPix& s, const L3dFastSrc& src, const float* h, Acc<COMP>& ss,
+    template <class P>
+    __device__ bool sums_tested(const P& s, const L3dFastSrc& src, const float* h, Acc<COMP>& ss,
                                 Acc<COMP>& sss, Acc<COMP>& srs) const {
         const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
-        const float2* win = exact_window();
 #pragma unroll 1
         for (int i = 0; i < S; i++) {
             const float x = s.px + (float)((i % 6) * 2 - 5), y = s.py + (float)((i / 6) * 2 - 5);
@@ -631,7 +621,7 @@ struct Exact {
             const float uu = qx * iz, vv = qy * iz;
             if (!(qz > 1e-6f) || !(uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax)) return false;
             const float val = bilinear_gather(src.tex, uu, vv);
-            const float2 rwv = win[i * XBLOCK];
+            const float2 rwv = s.win[i * P::kStride];
             ss.fma_add(rwv.x, val);
             const float wv = rwv.x * val;
             sss.fma_add(wv, val);
@@ -650,7 +640,8 @@ struct Exact {
      * what is left goes through sums_tested.  Bound by latency and issue: a test and a general
      * division per sample, each a branch that cuts a row's gathers apart, took 75.6 ms for four views
      * of 640x480 (8 sources, 5 iterations); this takes 39.2 ms. */
-    __device__ float view_cost(const XPix& s, const L3dFastSrc& src, const float* u) const {
+    template <class P>
+    __device__ float view_cost(const P& s, const L3dFastSrc& src, const float* u) const {
         float h[9];
 #pragma unroll
         for (int r = 0; r < 3; r++)
@@ -683,8 +674,7 @@ struct Exact {
         Acc<COMP> ss, sss, srs;
         if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv &&
             umax <= wmax - su && vmax <= hmax - sv) {
-            const float2* win = exact_window();
-#pragma unroll
+    #pragma unroll
             for (int r = 0; r < 6; r++) {
                 const float y = s.py + (float)(r * 2 - 5);
                 const float hz = fmaf(h[7], y, h[8]);
@@ -696,7 +686,7 @@ struct Exact {
                     const float x = s.px + (float)(c * 2 - 5);
                     const float iz = l3d_rcp_normal(fmaf(h[6], x, hz));
                     const float val = bilinear_gather(src.tex, fmaf(h[0], x, hx) * iz, fmaf(h[3], x, hy) * iz);
-                    const float2 rwv = win[i * XBLOCK];
+                    const float2 rwv = s.win[i * P::kStride];
                     const float w = rwv.x;
                     ss.fma_add(w, val);
                     const float wv = w * val;
@@ -717,14 +707,16 @@ struct Exact {
     }
 
     /* hypothesis_cost (patchmatch.wgsl.ts:192-233) */
-    __device__ float hypothesis_cost(const XPix& s, float3 n, float dd) const {
+    template <class P>
+    __device__ float cost_of(const P& s, float3 n, float dd) const {
         return hyp_cost(*this, v, d, s, n, dd);
     }
 
-    /* random_normal, random_depth (patchmatch.wgsl.ts:235-249) */
-    __device__ float3 random_normal(XPix& s) const {
-        float z = fmaf(random(s), 2.0f, -1.0f);
-        float a = random(s) * 6.2831853f;
+    /* random_normal (patchmatch.wgsl.ts:235-242) */
+    template <class P>
+    __device__ float3 random_normal(P& s) const {
+        float z = fmaf(l3d_random(&s.rng), 2.0f, -1.0f);
+        float a = l3d_random(&s.rng) * 6.2831853f;
         float r = sqrtf(maxw(0.0f, fmaf(-z, z, 1.0f)));
         float sn, cs;
         l3d_sincosf(a, &sn, &cs);
@@ -734,22 +726,23 @@ struct Exact {
         return normalize_ieee(make_float3(fmaf(view.x, -0.5f, n.x), fmaf(view.y, -0.5f, n.y),
                                           fmaf(view.z, -0.5f, n.z)));
     }
-    __device__ float random_depth(XPix& s) const {
-        float t = random(s);
-        return 1.0f / fmaf(v.range[0], t, v.range[1] * (1.0f - t));
-    }
-
-    __device__ void begin(XPix& s, int x, int y, int iteration, int phase) const {
-        s.px = (float)x;
-        s.py = (float)y;
-        uint32_t seed = (uint32_t)(v.ref + 1) * 0x9e3779b1u + (uint32_t)iteration * 97u +
-                        (uint32_t)phase * 13u + (v.flags & 1u) * 7u;
-        s.rng = l3d_pcg((uint32_t)(y * v.W + x) ^
-                        l3d_pcg(seed + (uint32_t)iteration * 7919u + (uint32_t)phase * 104729u));
-        prepare(s, x, y);
-        s.ray = ray_of(s.px, s.py);
-    }
 };
+
+/* The whole window of one pixel by one thread, in its column. */
+template <class E>
+__device__ __forceinline__ void thread_window(const E& f, typename E::template Pix<XBLOCK>& s, float2* win,
+                                              int x, int y) {
+    const float c = f.center(x, y);
+    typename E::Sums sums;
+#pragma unroll
+    for (int i = 0; i < S; i++) {
+        const float2 p = f.pair(x, y, i, c);
+        sums.add(p);
+        win[i * XBLOCK] = E::scale(p);
+    }
+    s.win = win;
+    f.finish(s, sums, c);
+}
 
 /* Block -> (view, tile) and the view's parameters in shared memory. */
 __device__ __forceinline__ int find_view(const L3dFastDev& d, int tile) {
@@ -773,23 +766,10 @@ __device__ __forceinline__ void load_view(L3dFastView& dst, const L3dFastView* s
     __syncthreads();
 }
 
-__device__ __forceinline__ void near_offset(int i, int* ox, int* oy) {
-    int m = (i + 1) / 2;
-    *ox = (i & 1) ? -m : m;
-    *oy = -(m + 1);
-}
-__device__ __forceinline__ void orient(int ox, int oy, int dir, int* rx, int* ry) {
-    switch (dir) {
-        case 1: *rx = ox; *ry = -oy; break;
-        case 2: *rx = oy; *ry = ox; break;
-        case 3: *rx = -oy; *ry = ox; break;
-        default: *rx = ox; *ry = oy; break;
-    }
-}
-
 template <class E>
 __global__ void __launch_bounds__(128) k_fast_init(const L3dFastDev d) {
     __shared__ __align__(16) L3dFastView sv;
+    __shared__ float2 windows[S * XBLOCK];
     load_view(sv, d.views + find_view(d, blockIdx.x));
     const int local = blockIdx.x - sv.tile_start;
     const int y = (local / sv.tiles_x) * TY + threadIdx.x / TX;
@@ -798,15 +778,16 @@ __global__ void __launch_bounds__(128) k_fast_init(const L3dFastDev d) {
     for (int half = 0; half < 2; half++) {
         const int xx = (local % sv.tiles_x) * (2 * TX) + (threadIdx.x % TX) * 2 + half;
         if (xx >= sv.W || y >= sv.H) continue;
-        typename E::Pix s;
+        typename E::template Pix<XBLOCK> s;
         f.begin(s, xx, y, 0, 0);
+        thread_window(f, s, windows + threadIdx.x, xx, y);
         const long long index = (long long)y * sv.W + xx;
         float3 n = f.random_normal(s);
         float dd = f.random_depth(s);
         if (sv.has_coarse && d.coarse) {
             /* init_coarse (patchmatch.wgsl.ts:296-333): the random plane against the planes of
              * the four nearest coarse pixels, re-intersected with this pixel's ray */
-            float c = f.hypothesis_cost(s, n, dd);
+            float c = f.cost_of(s, n, dd);
             const float qx = ((s.px + 0.5f) * (float)sv.cW) / (float)sv.W - 0.5f;
             const float qy = ((s.py + 0.5f) * (float)sv.cH) / (float)sv.H - 0.5f;
             const int bx = (int)floorf(qx), by = (int)floorf(qy);
@@ -821,7 +802,7 @@ __global__ void __launch_bounds__(128) k_fast_init(const L3dFastDev d) {
                 const float den = dot3f(hn, s.ray);
                 if (fabsf(den) < 1e-6f) continue;
                 const float hd = dot3f(hn, point) / den;
-                const float hc = f.hypothesis_cost(s, hn, hd);
+                const float hc = f.cost_of(s, hn, hd);
                 if (hc < c) {
                     c = hc;
                     n = hn;
@@ -839,13 +820,13 @@ __global__ void __launch_bounds__(128) k_fast_init(const L3dFastDev d) {
                 n = E::unpack_n(packed);
             }
         }
-        float c = f.hypothesis_cost(s, n, dd);
+        float c = f.cost_of(s, n, dd);
         if (!(sv.flags & 1u) && sv.has_prior) {
             float pd = d.prior[sv.pix_off + index];
             if (pd > 0.0f) {
                 float3 vv = E::normalize(s.ray);
                 float3 pn = make_float3(-vv.x, -vv.y, -vv.z);
-                float pc = f.hypothesis_cost(s, pn, pd);
+                float pc = f.cost_of(s, pn, pd);
                 if (pc < c) {
                     c = pc;
                     n = pn;
@@ -858,30 +839,25 @@ __global__ void __launch_bounds__(128) k_fast_init(const L3dFastDev d) {
     }
 }
 
-/* QUAD: the four lanes of each hardware quad take a 2 x 2 block of this colour's pixels (tighter
- * texture footprints per quad request); otherwise four consecutive pixels of one row. */
-template <class E, bool QUAD>
-__global__ void __launch_bounds__(128, E::kMinBlocks) k_fast_propagate(const L3dFastDev d, int iteration,
-                                                        int phase, float step) {
+/* propagate (patchmatch.wgsl.ts:349-423), one thread per pixel; the four lanes of each hardware quad
+ * take a 2 x 2 block of this colour's pixels (tighter texture footprints per quad request). */
+template <class E>
+__global__ void __launch_bounds__(128, E::kLayout.blocks) k_fast_propagate(const L3dFastDev d, int iteration,
+                                                                           int phase, float step) {
     __shared__ __align__(16) L3dFastView sv;
+    __shared__ float2 windows[S * XBLOCK];
     load_view(sv, d.views + find_view(d, blockIdx.x));
     if (iteration >= sv.iterations) return;
     const int local = blockIdx.x - sv.tile_start;
-    int tx, ty;
-    if (QUAD) {
-        const int q = threadIdx.x >> 2, j = threadIdx.x & 3;
-        tx = (q % (TX / 2)) * 2 + (j & 1);
-        ty = (q / (TX / 2)) * 2 + (j >> 1);
-    } else {
-        tx = threadIdx.x % TX;
-        ty = threadIdx.x / TX;
-    }
+    const int q = threadIdx.x >> 2, j = threadIdx.x & 3;
+    const int tx = (q % (TX / 2)) * 2 + (j & 1), ty = (q / (TX / 2)) * 2 + (j >> 1);
     const int y = (local / sv.tiles_x) * TY + ty;
     const int x = ((local % sv.tiles_x) * TX + tx) * 2 + ((y + phase) & 1);
     if (x >= sv.W || y >= sv.H) return;
     E f(sv, d);
-    typename E::Pix s;
+    typename E::template Pix<XBLOCK> s;
     f.begin(s, x, y, iteration, phase);
+    thread_window(f, s, windows + threadIdx.x, x, y);
     const int W = sv.W, H = sv.H;
     const long long base = sv.pix_off;
     const long long index = (long long)y * W + x;
@@ -890,23 +866,7 @@ __global__ void __launch_bounds__(128, E::kMinBlocks) k_fast_propagate(const L3d
     float bd = b.w;
     float best_cost = d.cost[base + index];
     for (int region = 0; region < 8; region++) {
-        const int count = region < 4 ? 7 : 11;
-        int chosen = -1;
-        float chosen_cost = 1e9f;
-        for (int i = 0; i < count; i++) {
-            int ox = 0, oy = -3 - 2 * i;
-            if (region < 4) near_offset(i, &ox, &oy);
-            int rx, ry;
-            orient(ox, oy, region & 3, &rx, &ry);
-            int qx = x + rx, qy = y + ry;
-            if (qx < 0 || qy < 0 || qx >= W || qy >= H) continue;
-            int qi = qy * W + qx;
-            float c = d.cost[base + qi];
-            if (c < chosen_cost) {
-                chosen_cost = c;
-                chosen = qi;
-            }
-        }
+        const int chosen = l3d_region_best(d.cost + base, region, x, y, W, H);
         if (chosen < 0) continue;
         float4 h = d.hyp[base + chosen];
         float3 hn = make_float3(h.x, h.y, h.z);
@@ -914,7 +874,7 @@ __global__ void __launch_bounds__(128, E::kMinBlocks) k_fast_propagate(const L3d
         float den = dot3f(hn, s.ray);
         if (fabsf(den) < 1e-6f) continue;
         float dd = dot3f(hn, make_float3(rq.x * h.w, rq.y * h.w, h.w)) / den;
-        float c = f.hypothesis_cost(s, hn, dd);
+        float c = f.cost_of(s, hn, dd);
         if (c < best_cost) {
             best_cost = c;
             bn = hn;
@@ -924,9 +884,9 @@ __global__ void __launch_bounds__(128, E::kMinBlocks) k_fast_propagate(const L3d
     float3 view = E::normalize(s.ray);
     float3 n_random = f.random_normal(s);
     float d_random = f.random_depth(s);
-    float e = (fmaf(f.random(s), 2.0f, -1.0f) * 0.15f) * step;
+    float e = (fmaf(l3d_random(&s.rng), 2.0f, -1.0f) * 0.15f) * step;
     float d_perturbed = 1.0f / ((1.0f / bd) * (1.0f + e));
-    float r1 = f.random(s), r2 = f.random(s), r3 = f.random(s);
+    float r1 = l3d_random(&s.rng), r2 = l3d_random(&s.rng), r3 = l3d_random(&s.rng);
     float3 n_perturbed = E::normalize(make_float3(bn.x + (fmaf(r1, 2.0f, -1.0f) * 0.6f) * step,
                                                     bn.y + (fmaf(r2, 2.0f, -1.0f) * 0.6f) * step,
                                                     bn.z + (fmaf(r3, 2.0f, -1.0f) * 0.6f) * step));
@@ -936,7 +896,7 @@ __global__ void __launch_bounds__(128, E::kMinBlocks) k_fast_propagate(const L3d
     for (int c = 0; c < 6; c++) {
         float3 nn = (c == 0 || c == 3) ? n_random : ((c == 1 || c == 5) ? n_perturbed : cur_n);
         float dv = (c == 0 || c == 2) ? d_random : ((c == 1 || c == 4) ? d_perturbed : cur_d);
-        float cand = f.hypothesis_cost(s, nn, dv);
+        float cand = f.cost_of(s, nn, dv);
         if (cand < best_cost) {
             best_cost = cand;
             bn = nn;
@@ -945,6 +905,45 @@ __global__ void __launch_bounds__(128, E::kMinBlocks) k_fast_propagate(const L3d
     }
     d.hyp[base + index] = make_float4(bn.x, bn.y, bn.z, bd);
     d.cost[base + index] = best_cost;
+}
+
+/* Blocks of 16 pixels, eight lanes each (l3d_lanes.cuh); a warp holds a 2 x 2 block of this
+ * colour's pixels. */
+constexpr int PARTS = TX * TY / 16;  /* blocks per tile of the propagate kernel */
+
+template <class E>
+__global__ void __launch_bounds__(128, E::kLayout.lane_blocks) k_fast_propagate_lanes(
+        const L3dFastDev d, int iteration, int phase, float step) {
+    __shared__ __align__(16) L3dFastView sv;
+    __shared__ float2 windows[S * 16];
+    const int tile = blockIdx.x / PARTS, part = blockIdx.x % PARTS;
+    load_view(sv, d.views + find_view(d, tile));
+    if (iteration >= sv.iterations) return;
+    const int local = tile - sv.tile_start;
+    const int warp = threadIdx.x >> 5, sub = (threadIdx.x >> 3) & 3, cand = threadIdx.x & 7;
+    const int ty = (part >> 1) * 2 + (sub >> 1), tx = (part & 1) * (TX / 2) + warp * 2 + (sub & 1);
+    int y = (local / sv.tiles_x) * TY + ty;
+    int x = ((local % sv.tiles_x) * TX + tx) * 2 + ((y + phase) & 1);
+    const bool inside = x < sv.W && y < sv.H;
+    if (!__any_sync(0xffffffffu, inside)) return;
+    x = min(x, sv.W - 1);  /* lanes outside the image stay for the shuffles and write nothing */
+    y = min(y, sv.H - 1);
+    E f(sv, d);
+    typename E::template Pix<1> s;
+    f.begin(s, x, y, iteration, phase);
+    float2* win = windows + (warp * 4 + sub) * S;
+    const float center = f.center(x, y);
+    for (int i = cand; i < S; i += 8) win[i] = f.pair(x, y, i, center);
+    __syncwarp();
+    typename E::Sums sums;
+#pragma unroll 6
+    for (int i = 0; i < S; i++) sums.add(win[i]);
+    f.finish(s, sums, center);
+    __syncwarp();
+    for (int i = cand; i < S; i += 8) win[i] = E::scale(win[i]);
+    __syncwarp();
+    s.win = win;
+    l3d_step_lanes(f, s, d.hyp + sv.pix_off, d.cost + sv.pix_off, x, y, sv.W, sv.H, inside, cand, step);
 }
 
 __global__ void k_fast_pack(const L3dFastDev d) {
@@ -962,6 +961,7 @@ template <class E>
 __global__ void __launch_bounds__(128) k_fast_plane_cost(const L3dFastDev d, const float4* planes,
                                                          float* cost) {
     __shared__ __align__(16) L3dFastView sv;
+    __shared__ float2 windows[S * XBLOCK];
     load_view(sv, d.views + find_view(d, blockIdx.x));
     const int local = blockIdx.x - sv.tile_start;
     const int y = (local / sv.tiles_x) * TY + threadIdx.x / TX;
@@ -969,11 +969,12 @@ __global__ void __launch_bounds__(128) k_fast_plane_cost(const L3dFastDev d, con
     for (int half = 0; half < 2; half++) {
         const int x = (local % sv.tiles_x) * (2 * TX) + (threadIdx.x % TX) * 2 + half;
         if (x >= sv.W || y >= sv.H) continue;
-        typename E::Pix s;
+        typename E::template Pix<XBLOCK> s;
         f.begin(s, x, y, 0, 0);
+        thread_window(f, s, windows + threadIdx.x, x, y);
         const long long index = (long long)y * sv.W + x;
         float4 p = planes[sv.pix_off + index];
-        cost[sv.pix_off + index] = f.hypothesis_cost(s, make_float3(p.x, p.y, p.z), p.w);
+        cost[sv.pix_off + index] = f.cost_of(s, make_float3(p.x, p.y, p.z), p.w);
     }
 }
 
@@ -981,13 +982,16 @@ __global__ void __launch_bounds__(128) k_fast_plane_cost(const L3dFastDev d, con
 
 namespace {
 
-template <class E, bool QUAD>
+template <class E>
 cudaError_t launch_eval(int kernel, const L3dFastDev& d, int iteration, int phase, cudaStream_t st) {
     if (kernel == L3D_K_INIT) {
         k_fast_init<E><<<d.total_tiles, 128, 0, st>>>(d);
     } else {
         float step = ldexpf(1.0f, -iteration);
-        k_fast_propagate<E, QUAD><<<d.total_tiles, 128, 0, st>>>(d, iteration, phase, step);
+        if (d.total_tiles <= E::kLayout.lane_tiles)
+            k_fast_propagate_lanes<E><<<d.total_tiles * PARTS, 128, 0, st>>>(d, iteration, phase, step);
+        else
+            k_fast_propagate<E><<<d.total_tiles, 128, 0, st>>>(d, iteration, phase, step);
     }
     return cudaGetLastError();
 }
@@ -1024,61 +1028,34 @@ cudaError_t l3d_launch_make_pairs(const void* img, int storage, int W, int H, ui
     return cudaGetLastError();
 }
 
-/* variant = texture rows (6, 4, 3, 2; the exact evaluator, compensated sums, gathers and the
- * shared window take 6 only) + 8 x quad mapping + 16 x texture gathers with exact weights (fast
- * evaluator, F16/F32/U8) + 32 x the reference window in shared memory (fast evaluator). */
+/* variant = texture rows (6, 4, 3, 2; the exact evaluator, compensated sums and gathers take 6
+ * only) + 16 x texture gathers with exact weights (fast evaluator, F16/F32/U8).  The quad (8) and
+ * shared-window (32) bits of earlier kernels select nothing any more: the propagate kernel always
+ * keeps the window in shared memory and a pixel's candidates in quads. */
 cudaError_t l3d_launch_fast(int kernel, const L3dFastDev& d, int iteration, int phase, int variant,
                             cudaStream_t stream) {
     if (d.total_tiles <= 0) return cudaSuccess;
     if (kernel != L3D_K_INIT && kernel != L3D_K_PROPAGATE) return cudaErrorInvalidValue;
     const int rows = variant & 7;
-    const bool quad = (variant & 8) != 0;
+    if (d.storage == 3 && !d.exact) { /* BF16 is sampled from linear memory */
+        if (d.comp) return launch_eval<Fast<false, 6, true>>(kernel, d, iteration, phase, stream);
+        return launch_eval<Fast<false, 6, false>>(kernel, d, iteration, phase, stream);
+    }
+    if (rows != 6 && (d.exact || d.comp || (variant & (16 | 32)) || !d.pairs)) return cudaErrorInvalidValue;
     if (d.exact) {
-        if (rows != 6) return cudaErrorInvalidValue;
-        if (d.comp) return quad ? launch_eval<Exact<true>, true>(kernel, d, iteration, phase, stream)
-                                : launch_eval<Exact<true>, false>(kernel, d, iteration, phase, stream);
-        return quad ? launch_eval<Exact<false>, true>(kernel, d, iteration, phase, stream)
-                    : launch_eval<Exact<false>, false>(kernel, d, iteration, phase, stream);
-    }
-    if (d.storage == 3) { /* BF16 is sampled from linear memory */
-        if (d.comp) return launch_eval<Fast<false, 6, true>, false>(kernel, d, iteration, phase, stream);
-        return launch_eval<Fast<false, 6, false>, false>(kernel, d, iteration, phase, stream);
-    }
-    if (variant & 32) { /* the reference window in shared memory (six texture rows) */
-        if (rows != 6) return cudaErrorInvalidValue;
-        switch ((d.comp ? 1 : 0) + ((variant & 16) ? 2 : 0) + (quad ? 4 : 0)) {
-            case 0: return launch_eval<Fast<true, 6, false, false, true>, false>(kernel, d, iteration, phase, stream);
-            case 1: return launch_eval<Fast<true, 6, true, false, true>, false>(kernel, d, iteration, phase, stream);
-            case 2: return launch_eval<Fast<true, 6, false, true, true>, false>(kernel, d, iteration, phase, stream);
-            case 3: return launch_eval<Fast<true, 6, true, true, true>, false>(kernel, d, iteration, phase, stream);
-            case 4: return launch_eval<Fast<true, 6, false, false, true>, true>(kernel, d, iteration, phase, stream);
-            case 5: return launch_eval<Fast<true, 6, true, false, true>, true>(kernel, d, iteration, phase, stream);
-            case 6: return launch_eval<Fast<true, 6, false, true, true>, true>(kernel, d, iteration, phase, stream);
-            default: return launch_eval<Fast<true, 6, true, true, true>, true>(kernel, d, iteration, phase, stream);
-        }
+        if (d.comp) return launch_eval<Exact<true>>(kernel, d, iteration, phase, stream);
+        return launch_eval<Exact<false>>(kernel, d, iteration, phase, stream);
     }
     if (variant & 16) { /* texture gathers with exact weights */
-        if (rows != 6) return cudaErrorInvalidValue;
-        if (d.comp) return quad ? launch_eval<Fast<true, 6, true, true>, true>(kernel, d, iteration, phase, stream)
-                                : launch_eval<Fast<true, 6, true, true>, false>(kernel, d, iteration, phase, stream);
-        return quad ? launch_eval<Fast<true, 6, false, true>, true>(kernel, d, iteration, phase, stream)
-                    : launch_eval<Fast<true, 6, false, true>, false>(kernel, d, iteration, phase, stream);
+        if (d.comp) return launch_eval<Fast<true, 6, true, true>>(kernel, d, iteration, phase, stream);
+        return launch_eval<Fast<true, 6, false, true>>(kernel, d, iteration, phase, stream);
     }
-    if (d.comp) {
-        if (rows != 6) return cudaErrorInvalidValue;
-        return quad ? launch_eval<Fast<true, 6, true>, true>(kernel, d, iteration, phase, stream)
-                    : launch_eval<Fast<true, 6, true>, false>(kernel, d, iteration, phase, stream);
-    }
-    if (!d.pairs && rows < 6) return cudaErrorInvalidValue;
-    switch (rows + (quad ? 8 : 0)) {
-        case 6: return launch_eval<Fast<true, 6>, false>(kernel, d, iteration, phase, stream);
-        case 4: return launch_eval<Fast<true, 4>, false>(kernel, d, iteration, phase, stream);
-        case 3: return launch_eval<Fast<true, 3>, false>(kernel, d, iteration, phase, stream);
-        case 2: return launch_eval<Fast<true, 2>, false>(kernel, d, iteration, phase, stream);
-        case 14: return launch_eval<Fast<true, 6>, true>(kernel, d, iteration, phase, stream);
-        case 12: return launch_eval<Fast<true, 4>, true>(kernel, d, iteration, phase, stream);
-        case 11: return launch_eval<Fast<true, 3>, true>(kernel, d, iteration, phase, stream);
-        case 10: return launch_eval<Fast<true, 2>, true>(kernel, d, iteration, phase, stream);
+    if (d.comp) return launch_eval<Fast<true, 6, true>>(kernel, d, iteration, phase, stream);
+    switch (rows) {
+        case 6: return launch_eval<Fast<true, 6>>(kernel, d, iteration, phase, stream);
+        case 4: return launch_eval<Fast<true, 4>>(kernel, d, iteration, phase, stream);
+        case 3: return launch_eval<Fast<true, 3>>(kernel, d, iteration, phase, stream);
+        case 2: return launch_eval<Fast<true, 2>>(kernel, d, iteration, phase, stream);
         default: return cudaErrorInvalidValue;
     }
 }

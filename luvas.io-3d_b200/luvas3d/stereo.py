@@ -294,8 +294,8 @@ class DenseStereo:
 
     @property
     def variant(self) -> int:
-        """Batched-form kernel variant: texture-sampled window rows + 8 x quad lane mapping
-        + 16 x texture gathers with exact weights + 32 x the window in shared memory."""
+        """Batched-form kernel variant: texture-sampled window rows + 16 x texture gathers with exact
+        weights (+ 8 and + 32 are accepted and select nothing)."""
         return int(self._lib.l3d_stereo_variant(self._h()))
 
     @variant.setter
