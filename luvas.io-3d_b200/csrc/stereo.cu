@@ -19,9 +19,9 @@
 #include <stdint.h>
 
 #include "l3d_fmath.h"
-#include "l3d_ieee.h"
 #include "l3d_internal.h"
 #include "l3d_lanes.cuh"
+#include "l3d_window.cuh"
 
 namespace {
 
@@ -205,13 +205,9 @@ struct Stereo {
     }
 
     /* view_cost (patchmatch.wgsl.ts:130-159); a sample with q.z <= 1e-6 or outside the image makes the
-     * cost 2.  The window's image is the convex hull of its corners' images, so four corners inside
-     * by more than the rounding of a position (`slack`, from the magnitudes that enter it: each of
-     * q's components carries three roundings, the quotient two more, and the bound allows sixteen)
-     * stand for every sample, and their loop is straight-line code without tests; a corner outside
-     * by as much rejects the window at once; the rest goes through sums_tested.  One view of
-     * 640x480, 8 sources, 5 iterations: 13.4 ms; a test and a general division per sample, with the
-     * window in registers, took 38.4 ms. */
+     * cost 2 (l3d_window.cuh).  A window inside the image runs as straight-line code: one view of
+     * 640x480, 8 sources, 5 iterations took 38.4 ms with a test and a general division per sample and
+     * the window in registers, 13.4 ms without. */
     template <class P>
     __device__ float view_cost(const P& s, const L3dSrc& src, const float* u) const {
         float h[9];
@@ -219,43 +215,25 @@ struct Stereo {
         for (int r = 0; r < 3; r++)
 #pragma unroll
             for (int c = 0; c < 3; c++) h[r * 3 + c] = fmaf(src.kt[r], u[c], src.B[r * 3 + c]);
-        const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
-        constexpr float E = (float)W_::HALF;
-        float zmin = 3.0e38f, zmax = -3.0e38f, umin = 3.0e38f, umax = -3.0e38f, vmin = 3.0e38f, vmax = -3.0e38f;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const float x = s.px + ((c & 1) ? E : -E);
-            const float y = s.py + ((c & 2) ? E : -E);
-            const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
-            const float iz = l3d_rcp_approx(qz);
-            const float uu = fmaf(h[0], x, fmaf(h[1], y, h[2])) * iz;
-            const float vv = fmaf(h[3], x, fmaf(h[4], y, h[5])) * iz;
-            zmin = fminf(zmin, qz);
-            zmax = fmaxf(zmax, qz);
-            umin = fminf(umin, uu);
-            umax = fmaxf(umax, uu);
-            vmin = fminf(vmin, vv);
-            vmax = fmaxf(vmax, vv);
-        }
-        const float ax = s.px + E, ay = s.py + E;
-        const float mz = fmaf(fabsf(h[6]), ax, fmaf(fabsf(h[7]), ay, fabsf(h[8])));
-        const float mx = fmaf(fabsf(h[0]), ax, fmaf(fabsf(h[1]), ay, fabsf(h[2])));
-        const float my = fmaf(fabsf(h[3]), ax, fmaf(fabsf(h[4]), ay, fabsf(h[5])));
-        const float unit = 0x1p-20f * l3d_rcp_approx(zmin);
-        const float su = unit * fmaf(wmax, mz, mx), sv = unit * fmaf(hmax, mz, my);
+        const L3dPlace place =
+            l3d_window_place(h, s.px, s.py, (float)W_::HALF, (float)(src.W - 1), (float)(src.H - 1));
         Sums sum = {0.0f, 0.0f, 0.0f};
-        if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv &&
-            umax <= wmax - su && vmax <= hmax - sv) {
+        if (place == L3D_INSIDE) {
+            /* rows rolled: all 36 samples in a line overflow the instruction cache (11.0 against
+             * 12.8 ms for the view above) */
+#pragma unroll 1
+            for (int row = 0; row < N; row++) {
+                const float y = s.py + (float)W_::oy(row * N);
 #pragma unroll
-            for (int i = 0; i < W_::S; i++) {
-                const float x = s.px + (float)W_::ox(i), y = s.py + (float)W_::oy(i);
-                const float iz = l3d_rcp_normal(fmaf(h[6], x, fmaf(h[7], y, h[8])));
-                const float uu = fmaf(h[0], x, fmaf(h[1], y, h[2])) * iz;
-                const float vv = fmaf(h[3], x, fmaf(h[4], y, h[5])) * iz;
-                sum.add(s.win.get(i), bilinear<true>(src, uu, vv));
+                for (int col = 0; col < N; col++) {
+                    const float x = s.px + (float)W_::ox(col);
+                    const float iz = l3d_rcp_normal(fmaf(h[6], x, fmaf(h[7], y, h[8])));
+                    const float uu = fmaf(h[0], x, fmaf(h[1], y, h[2])) * iz;
+                    const float vv = fmaf(h[3], x, fmaf(h[4], y, h[5])) * iz;
+                    sum.add(s.win.get(row * N + col), bilinear<true>(src, uu, vv));
+                }
             }
-        } else if (zmin <= 1e-6f || umin < -su || vmin < -sv || umax > wmax + su || vmax > hmax + sv ||
-                   !sums_tested(s, src, h, sum)) {
+        } else if (place == L3D_OUTSIDE || !sums_tested(s, src, h, sum)) {
             return 2.0f;
         }
         float mean = sum.ss / s.rsum;
@@ -464,12 +442,13 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
 
 /* propagate (patchmatch.wgsl.ts:349-423), eight lanes per pixel (l3d_lanes.cuh): a warp holds a 2 x 2
  * block of the colour's pixels, a block 8 x 2.  Bound by issue and the latency of the sample loads, so
- * resident warps pay more than registers: seven blocks per SM (the 6 x 6 window at 640x480, 8
- * sources, 3 iterations: 4 blocks 9.1 ms, 5 8.3, 7 8.15, 8 8.2, 10 9.3).  A thread per pixel with the
- * window in a shared-memory column took 8.4 ms there, 38.8 against 36.2 ms at 1280x960 and 1.6
- * against 0.61 ms at 160x120, so no size keeps it.  The dense 11 x 11 window, whose pairs a thread alone
- * keeps in local memory, went from 53.7 to 13.0 ms at 640x480 (4 sources, 2 iterations). */
-constexpr int kPropagateBlocks = 7;
+ * resident warps pay more than registers: six blocks per SM (the 6 x 6 window, 640x480, 8 sources, 5
+ * iterations: 6 blocks 11.0 ms, 8 10.9, 10 11.5; 160x120, 4 sources, 3 iterations: 0.41, 0.43, 0.45).
+ * A thread per pixel with the window in a shared-memory column was slower at every size (160x120 0.96
+ * ms against 0.41, 640x480 13.4 against 12.8 and 1280x960 38.8 against 36.2 with the samples unrolled
+ * in both).  The dense 11 x 11 window, whose pairs a thread alone keeps in local memory, went from
+ * 53.7 to 9.7 ms at 640x480 (4 sources, 2 iterations). */
+constexpr int kPropagateBlocks = 6;
 template <int N, int DIL>
 __global__ void __launch_bounds__(128, kPropagateBlocks) k_propagate(const L3dParams p, const L3dStereoDev d) {
     __shared__ float2 windows[N * N * 16];

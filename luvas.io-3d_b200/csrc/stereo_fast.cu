@@ -39,9 +39,9 @@
 #include <cuda_fp16.h>
 
 #include "l3d_fmath.h"
-#include "l3d_ieee.h"
 #include "l3d_internal.h"
 #include "l3d_lanes.cuh"
+#include "l3d_window.cuh"
 
 namespace {
 
@@ -64,7 +64,7 @@ constexpr Layout kFilter = {5, 5, 3000};
 constexpr Layout kGather = {4, 5, 1000};
 /* The exact evaluator likewise: 2.13 / 1.72, 4.41 / 3.77, 6.47 / 6.81.  With four blocks the compiler
  * has the registers to keep a row's gathers in flight, which is worth more than warps (four views,
- * 5 iterations, thread per pixel: 4 blocks 39.2 ms, 5 47.2 ms, 6 57.5 ms). */
+ * 5 iterations, thread per pixel: 3 blocks 35.6 ms, 4 35.9 ms, 5 38.9 ms). */
 constexpr Layout kExact = {4, 4, 1000};
 
 __device__ __forceinline__ float dot3f(float3 a, float3 b) {
@@ -410,6 +410,10 @@ template <bool TEX, int TEXROWS = 6, bool COMP = false, bool GATHER = false>
 struct Fast : Scene {
     template <int STRIDE> using Pix = FPix<STRIDE>;
     static constexpr Layout kLayout = GATHER ? kGather : kFilter;
+    /* window rows unrolled together: filtered samples want all their fetches in flight, a gather's
+     * row of blends is long enough that more than two overflow the instruction cache (four views of
+     * 640x480, 8 sources, 5 iterations: 33.6 ms, all six rows 34.6; filtered 23.9 and 23.6) */
+    static constexpr int kRows = GATHER ? 2 : 6;
     using Scene::Scene;
 
     static __device__ __forceinline__ float3 normalize(float3 a) { return normalize_fast(a); }
@@ -485,7 +489,7 @@ struct Fast : Scene {
          * fetches in flight together */
         constexpr int RT = TEX ? TEXROWS : 6;
         float rx = qx0, ry = qy0, rz = qz0;
-#pragma unroll
+#pragma unroll kRows
         for (int r = 0; r < RT; r++) {
             float qx = rx, qy = ry, qz = rz;
 #pragma unroll
@@ -632,14 +636,10 @@ struct Exact : Scene {
 
     /* view_cost (patchmatch.wgsl.ts:130-159) with H = B + kt u^T (Bt/ktt hold the unshifted
      * base in this form).  Every sample is computed as the oracle computes it; a sample with
-     * q.z <= 1e-6 or outside [0, W-1] x [0, H-1] makes the cost 2.  The window's image is the convex
-     * hull of its corners' images, so four corners inside by more than the rounding of a position
-     * (`slack`, from the magnitudes that enter it: each of q's components carries three roundings,
-     * the quotient two more, and the bound allows sixteen) stand for all 36 samples: their loop is
-     * straight-line code without tests.  A window with a corner outside by as much costs 2 at once;
-     * what is left goes through sums_tested.  Bound by latency and issue: a test and a general
-     * division per sample, each a branch that cuts a row's gathers apart, took 75.6 ms for four views
-     * of 640x480 (8 sources, 5 iterations); this takes 39.2 ms. */
+     * q.z <= 1e-6 or outside [0, W-1] x [0, H-1] makes the cost 2 (l3d_window.cuh).  Bound by latency
+     * and issue: a test and a general division per sample, each a branch that cuts a row's gathers
+     * apart, took 75.6 ms for four views of 640x480 (8 sources, 5 iterations); the straight line for
+     * windows inside the image takes 35.9 ms. */
     template <class P>
     __device__ float view_cost(const P& s, const L3dFastSrc& src, const float* u) const {
         float h[9];
@@ -647,34 +647,12 @@ struct Exact : Scene {
         for (int r = 0; r < 3; r++)
 #pragma unroll
             for (int c = 0; c < 3; c++) h[r * 3 + c] = fmaf(src.ktt[r], u[c], src.Bt[r * 3 + c]);
-        const float wmax = (float)(src.W - 1), hmax = (float)(src.H - 1);
-        float zmin = 3.0e38f, zmax = -3.0e38f, umin = 3.0e38f, umax = -3.0e38f, vmin = 3.0e38f, vmax = -3.0e38f;
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const float x = s.px + ((c & 1) ? 5.0f : -5.0f);
-            const float y = s.py + ((c & 2) ? 5.0f : -5.0f);
-            const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
-            const float qx = fmaf(h[0], x, fmaf(h[1], y, h[2]));
-            const float qy = fmaf(h[3], x, fmaf(h[4], y, h[5]));
-            const float iz = l3d_rcp_approx(qz);
-            const float uu = qx * iz, vv = qy * iz;
-            zmin = fminf(zmin, qz);
-            zmax = fmaxf(zmax, qz);
-            umin = fminf(umin, uu);
-            umax = fmaxf(umax, uu);
-            vmin = fminf(vmin, vv);
-            vmax = fmaxf(vmax, vv);
-        }
-        const float ax = fabsf(s.px) + 5.0f, ay = fabsf(s.py) + 5.0f;
-        const float mz = fmaf(fabsf(h[6]), ax, fmaf(fabsf(h[7]), ay, fabsf(h[8])));
-        const float mx = fmaf(fabsf(h[0]), ax, fmaf(fabsf(h[1]), ay, fabsf(h[2])));
-        const float my = fmaf(fabsf(h[3]), ax, fmaf(fabsf(h[4]), ay, fabsf(h[5])));
-        const float unit = 0x1p-20f * l3d_rcp_approx(zmin);
-        const float su = unit * fmaf(wmax, mz, mx), sv = unit * fmaf(hmax, mz, my);
+        const L3dPlace place =
+            l3d_window_place(h, s.px, s.py, 5.0f, (float)(src.W - 1), (float)(src.H - 1));
         Acc<COMP> ss, sss, srs;
-        if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv &&
-            umax <= wmax - su && vmax <= hmax - sv) {
-    #pragma unroll
+        if (place == L3D_INSIDE) {
+            /* rows rolled: unrolled they overflow the instruction cache (35.9 against 38.8 ms) */
+#pragma unroll 1
             for (int r = 0; r < 6; r++) {
                 const float y = s.py + (float)(r * 2 - 5);
                 const float hz = fmaf(h[7], y, h[8]);
@@ -694,8 +672,7 @@ struct Exact : Scene {
                     srs.fma_add(wv, rwv.y);
                 }
             }
-        } else if (zmin <= 1e-6f || umin < -su || vmin < -sv || umax > wmax + su || vmax > hmax + sv ||
-                   !sums_tested(s, src, h, ss, sss, srs)) {
+        } else if (place == L3D_OUTSIDE || !sums_tested(s, src, h, ss, sss, srs)) {
             return 2.0f;
         }
         const float mean = ss.value() / s.rsum;
