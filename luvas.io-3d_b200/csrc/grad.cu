@@ -21,6 +21,8 @@
  *   e_i = (u . x_i) K_s^T dc/dq       the gradient at the source-camera point
  *                                     Y_i = K_s^-1 q / (u . x_i)
  *   S1 += e_i,  S2 += Y_i x e_i       summed per (reference, source) pair over all pixels
+ * Both are bilinear in g_i = dc/dq and x_i (u . x_i cancels in Y_i x e_i), so a window's S1 and S2
+ * follow from sum g_i and its moments sum g_i x_i^T, taken about the centre pixel.
  * k_finalize turns S1 and S2 into the gradients of both views' increments in FP64 with the
  * exact SO(3) left Jacobians; k_compose builds each pair's relative pose and homography base
  * from the FP64 base poses and the increments, in FP64 on the device.  The warped samples are
@@ -34,6 +36,7 @@
 #include "../../include/luvas3d.h"
 #include "l3d_fmath.h"
 #include "l3d_internal.h"
+#include "l3d_window.cuh"
 
 namespace {
 
@@ -174,25 +177,49 @@ __device__ __forceinline__ float texel(const void* img, long long i) {
     if (ST == L3D_DTYPE_F32) return __ldg((const float*)img + i);
     if (ST == L3D_DTYPE_F16) return __half2float(__ldg((const __half*)img + i));
     if (ST == L3D_DTYPE_BF16) return __bfloat162float(__ldg((const __nv_bfloat16*)img + i));
-    return (float)__ldg((const uint8_t*)img + i) / 255.0f;
+    /* u / 255 rounded: the quotient of l3d_div_normal with the divisor's reciprocal written out */
+    const float u = (float)__ldg((const uint8_t*)img + i), q = u * 0x1.010102p-8f;
+    return fmaf(fmaf(-255.0f, q, u), 0x1.010102p-8f, q);
 }
 
-/* Bilinear sample (clamp to edge) at texel coordinates (u, v) and its gradient. */
-template <int ST>
+/* Bilinear sample (clamp to edge) at texel coordinates (u, v) and its gradient.  INSIDE: the
+ * footprint lies in the image, nothing is clamped. */
+template <int ST, bool INSIDE>
 __device__ __forceinline__ float bilinear_grad(const void* img, int W, int H, float u, float v,
                                                float* gu, float* gv) {
     const float x0f = floorf(u), y0f = floorf(v);
     const float fx = u - x0f, fy = v - y0f;
-    const int x0 = min(max((int)x0f, 0), W - 1), y0 = min(max((int)y0f, 0), H - 1);
-    const int x1 = min(x0 + 1, W - 1), y1 = min(y0 + 1, H - 1);
-    const float a = texel<ST>(img, (long long)y0 * W + x0);
-    const float b = texel<ST>(img, (long long)y0 * W + x1);
-    const float c = texel<ST>(img, (long long)y1 * W + x0);
-    const float e = texel<ST>(img, (long long)y1 * W + x1);
+    int x0 = (int)x0f, y0 = (int)y0f, dx = 1, dy = W;
+    if (!INSIDE) {
+        x0 = min(max(x0, 0), W - 1);
+        y0 = min(max(y0, 0), H - 1);
+        dx = x0 + 1 < W ? 1 : 0;
+        dy = y0 + 1 < H ? W : 0;
+    }
+    const long long i = y0 * W + x0;
+    const float a = texel<ST>(img, i);
+    const float b = texel<ST>(img, i + dx);
+    const float c = texel<ST>(img, i + dy);
+    const float e = texel<ST>(img, i + dy + dx);
     const float top = fmaf(fx, b - a, a), bot = fmaf(fx, e - c, c);
     *gu = fmaf(fy, (e - c) - (b - a), b - a);
     *gv = bot - top;
     return fmaf(fy, bot - top, top);
+}
+
+/* One warped sample of a window: its position, value and image gradient. */
+struct Sample {
+    float iz, u, v, val, gx, gy;
+};
+template <int ST, bool INSIDE>
+__device__ __forceinline__ Sample warp_sample(const L3dGradPair& pr, const void* img, const float* h, float x, float y) {
+    Sample s;
+    const float qz = fmaf(h[6], x, fmaf(h[7], y, h[8]));
+    s.iz = INSIDE ? l3d_rcp_normal(qz) : 1.0f / qz;
+    s.u = fmaf(h[0], x, fmaf(h[1], y, h[2])) * s.iz;
+    s.v = fmaf(h[3], x, fmaf(h[4], y, h[5])) * s.iz;
+    s.val = bilinear_grad<ST, INSIDE>(img, pr.W, pr.H, s.u, s.v, &s.gx, &s.gy);
+    return s;
 }
 
 constexpr int kTileX = 32, kTileY = 4;
@@ -200,7 +227,10 @@ constexpr int kTileX = 32, kTileY = 4;
 /* One thread per reference pixel, blocks of 32 x 4 pixels.  Each (pixel, source) pair takes
  * one pass over the window for the statistics and, when gradients are wanted, a second pass
  * that recomputes the samples and pushes the gradient through them.  Per-pair sums S1, S2 are
- * reduced per block and added to pair_sums in FP64. */
+ * reduced per block and added to pair_sums in FP64.  Bound by issue: windows inside the image run
+ * without per-sample tests, clamps or general divisions (l3d_window.cuh), and the pose's sums come
+ * from nine sums of g and its moments about the centre instead of a source-camera point, a cross
+ * product and a division per sample.  Three views of 640x480, 4 sources: 1304 -> 637 us. */
 template <int N, int DIL, int ST>
 __global__ void __launch_bounds__(kTileX * kTileY) k_ncc_grad(
         const L3dGradDev d, const L3dGradPair* __restrict__ pairs, int n,
@@ -219,15 +249,14 @@ __global__ void __launch_bounds__(kTileX * kTileY) k_ncc_grad(
     const float px = (float)x, py = (float)y;
 
     /* reference window: values and bilateral weights (prepare_window) */
-    /* the reference window in shared memory (lane-major) when it fits: the gradient pass
-     * indexes it in a loop that is not fully unrolled, which puts register arrays in local
-     * memory; the 11 x 11 window stays in (local) per-thread arrays */
+    /* pairs (w, r), a column of shared memory per thread when the window fits (the loops over its rows
+     * index it, which would put register arrays in local memory); the 11 x 11 window stays in local
+     * per-thread arrays */
     constexpr bool kSharedWin = S <= 36;
     constexpr int LS = kSharedWin ? kTileX * kTileY : 1;
-    __shared__ float rv_s[kSharedWin ? S : 1][kTileX * kTileY], rw_s[kSharedWin ? S : 1][kTileX * kTileY];
-    float rv_l[kSharedWin ? 1 : S], rw_l[kSharedWin ? 1 : S];
-    float* const rv = kSharedWin ? &rv_s[0][threadIdx.x] : rv_l;
-    float* const rw = kSharedWin ? &rw_s[0][threadIdx.x] : rw_l;
+    __shared__ float2 win_s[kSharedWin ? S * LS : 1];
+    float2 win_l[kSharedWin ? 1 : S];
+    float2* const win = kSharedWin ? win_s + threadIdx.x : win_l;
     float rsum = 1.0f, rmean = 0.0f, rvar = 0.0f;
     if (active) {
         const float center = texel<ST>(d.images, d.ref_img_off + idx);
@@ -240,8 +269,7 @@ __global__ void __launch_bounds__(kTileX * kTileY) k_ncc_grad(
             const float dc = v - center;
             const float wgt = l3d_expf(-(dc * dc) / (2.0f * 0.06f * 0.06f) -
                                        (float)(ox * ox + oy * oy) / (2.0f * 5.0f * 5.0f));
-            rv[i * LS] = v;
-            rw[i * LS] = wgt;
+            win[i * LS] = make_float2(wgt, v);
             sw = sw + wgt;
             sr = fmaf(wgt, v, sr);
             srr = fmaf(wgt * v, v, srr);
@@ -286,25 +314,40 @@ __global__ void __launch_bounds__(kTileX * kTileY) k_ncc_grad(
                 h[r * 3 + 2] = fmaf(pr.kt[r], u2, pr.B[r * 3 + 2]);
             }
             const void* img = (const char*)d.images + pr.img_off * d.elem;
-            const float wmax = (float)(pr.W - 1), hmax = (float)(pr.H - 1);
-            bool ok = true;
+            const L3dPlace place =
+                l3d_window_place(h, px, py, (float)HALF, (float)(pr.W - 1), (float)(pr.H - 1));
+            bool ok = place == L3D_INSIDE;
             float ss = 0.0f, sss = 0.0f, srs = 0.0f;
-#pragma unroll
-            for (int i = 0; i < S; i++) {
-                const float xi = px + (float)((i % N) * DIL - HALF);
-                const float yi = py + (float)((i / N) * DIL - HALF);
-                const float qz = fmaf(h[6], xi, fmaf(h[7], yi, h[8]));
-                const float qx = fmaf(h[0], xi, fmaf(h[1], yi, h[2]));
-                const float qy = fmaf(h[3], xi, fmaf(h[4], yi, h[5]));
-                const float iz = 1.0f / qz;
-                const float uu = qx * iz, vv = qy * iz;
-                ok = ok && qz > 1e-6f && uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax;
-                float gx, gy;
-                const float val = ok ? bilinear_grad<ST>(img, pr.W, pr.H, uu, vv, &gx, &gy) : 0.0f;
-                ss = fmaf(rw[i * LS], val, ss);
-                const float wv = rw[i * LS] * val;
+            auto add = [&](float2 p, float val) {
+                ss = fmaf(p.x, val, ss);
+                const float wv = p.x * val;
                 sss = fmaf(wv, val, sss);
-                srs = fmaf(wv, rv[i * LS], srs);
+                srs = fmaf(wv, p.y, srs);
+            };
+            if (ok) {
+                /* rows rolled here and below: unrolled, the samples overflow the instruction cache (660
+                 * us for the views quoted above) */
+#pragma unroll 1
+                for (int row = 0; row < N; row++) {
+                    const float yi = py + (float)(row * DIL - HALF);
+#pragma unroll
+                    for (int col = 0; col < N; col++)
+                        add(win[(row * N + col) * LS],
+                            warp_sample<ST, true>(pr, img, h, px + (float)(col * DIL - HALF), yi).val);
+                }
+            } else if (place == L3D_GRAZES) {
+                ok = true;
+                const float wmax = (float)(pr.W - 1), hmax = (float)(pr.H - 1);
+#pragma unroll 1
+                for (int i = 0; i < S && ok; i++) {
+                    const float xi = px + (float)((i % N) * DIL - HALF), yi = py + (float)((i / N) * DIL - HALF);
+                    const float qz = fmaf(h[6], xi, fmaf(h[7], yi, h[8]));
+                    const float iz = 1.0f / qz;
+                    const float uu = fmaf(h[0], xi, fmaf(h[1], yi, h[2])) * iz;
+                    const float vv = fmaf(h[3], xi, fmaf(h[4], yi, h[5])) * iz;
+                    ok = qz > 1e-6f && uu >= 0.0f && vv >= 0.0f && uu <= wmax && vv <= hmax;
+                    if (ok) add(win[i * LS], warp_sample<ST, false>(pr, img, h, xi, yi).val);
+                }
             }
             if (ok) {
                 const float ms = ss / rsum;
@@ -319,45 +362,76 @@ __global__ void __launch_bounds__(kTileX * kTileY) k_ncc_grad(
                     c = fminf(fmaxf(raw, 0.0f), 2.0f);
                     if (want_grad && raw > 0.0f && raw < 2.0f) {
                         const float inv_w = 1.0f / rsum, iden = 1.0f / den, ivs = 1.0f / vs;
-                        const float ks0 = pr.ks[0], ks1 = pr.ks[1], ks2 = pr.ks[2], ks3 = pr.ks[3];
-                        const float iks0 = 1.0f / ks0, iks1 = 1.0f / ks1;
                         const float kt0 = pr.kt[0], kt1 = pr.kt[1], kt2 = pr.kt[2];
-#pragma unroll 4
-                        for (int i = 0; i < S; i++) {
-                            const float xi = px + (float)((i % N) * DIL - HALF);
-                            const float yi = py + (float)((i / N) * DIL - HALF);
-                            const float qz = fmaf(h[6], xi, fmaf(h[7], yi, h[8]));
-                            const float qx = fmaf(h[0], xi, fmaf(h[1], yi, h[2]));
-                            const float qy = fmaf(h[3], xi, fmaf(h[4], yi, h[5]));
-                            const float iz = 1.0f / qz;
-                            const float uu = qx * iz, vv = qy * iz;
-                            float gx, gy;
-                            const float val = bilinear_grad<ST>(img, pr.W, pr.H, uu, vv, &gx, &gy);
-                            const float dcs = -gout * (rw[i * LS] * inv_w) *
-                                              ((rv[i * LS] - rmean) * iden - ncc * (val - ms) * ivs);
-                            const float g0 = dcs * iz * gx, g1 = dcs * iz * gy;
-                            const float g2 = -(g0 * uu + g1 * vv);
-                            /* plane */
+                        /* sums of g = dL/dq over the window, of g x' and of g y', (x', y') the sample's
+                         * offset from the centre: the pose's gradients follow from them */
+                        float t0 = 0.0f, t1 = 0.0f, t2 = 0.0f, x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
+                        float y0 = 0.0f, y1 = 0.0f, y2 = 0.0f;
+                        auto push = [&](float2 p, const Sample& q, float xi, float yi, float ox, float& r0,
+                                        float& r1, float& r2) {
+                            const float dcs = -gout * (p.x * inv_w) *
+                                              ((p.y - rmean) * iden - ncc * (q.val - ms) * ivs);
+                            const float g0 = dcs * q.iz * q.gx, g1 = dcs * q.iz * q.gy;
+                            const float g2 = -(g0 * q.u + g1 * q.v);
+                            r0 += g0;
+                            r1 += g1;
+                            r2 += g2;
+                            x0 = fmaf(g0, ox, x0);
+                            x1 = fmaf(g1, ox, x1);
+                            x2 = fmaf(g2, ox, x2);
                             const float a = fmaf(g0, kt0, fmaf(g1, kt1, g2 * kt2));
                             gu0 = fmaf(a, xi, gu0);
                             gu1 = fmaf(a, yi, gu1);
                             gu2 += a;
-                            /* pose: e = lambda K_s^T g at Y = K_s^-1 q / lambda */
-                            const float lam = fmaf(u0, xi, fmaf(u1, yi, u2));
-                            const float e0 = lam * (ks0 * g0);
-                            const float e1 = lam * (ks1 * g1);
-                            const float e2 = lam * fmaf(ks2, g0, fmaf(ks3, g1, g2));
-                            const float il = 1.0f / lam;
-                            const float Y2 = qz * il;
-                            const float Y0 = (fmaf(-ks2, qz, qx) * iks0) * il;
-                            const float Y1 = (fmaf(-ks3, qz, qy) * iks1) * il;
-                            S1x += e0;
-                            S1y += e1;
-                            S1z += e2;
-                            S2x += Y1 * e2 - Y2 * e1;
-                            S2y += Y2 * e0 - Y0 * e2;
-                            S2z += Y0 * e1 - Y1 * e0;
+                        };
+#pragma unroll 1
+                        for (int row = 0; row < N; row++) {
+                            const float oy = (float)(row * DIL - HALF), yi = py + oy;
+                            float r0 = 0.0f, r1 = 0.0f, r2 = 0.0f;
+                            if (place == L3D_INSIDE) {
+#pragma unroll
+                                for (int col = 0; col < N; col++) {
+                                    const float ox = (float)(col * DIL - HALF);
+                                    push(win[(row * N + col) * LS], warp_sample<ST, true>(pr, img, h, px + ox, yi),
+                                         px + ox, yi, ox, r0, r1, r2);
+                                }
+                            } else {
+#pragma unroll 1
+                                for (int col = 0; col < N; col++) {
+                                    const float ox = (float)(col * DIL - HALF);
+                                    push(win[(row * N + col) * LS], warp_sample<ST, false>(pr, img, h, px + ox, yi),
+                                         px + ox, yi, ox, r0, r1, r2);
+                                }
+                            }
+                            t0 += r0;
+                            t1 += r1;
+                            t2 += r2;
+                            y0 = fmaf(r0, oy, y0);
+                            y1 = fmaf(r1, oy, y1);
+                            y2 = fmaf(r2, oy, y2);
                         }
+                        /* pose: S1 = K_s^T sum lambda g, lambda = u . (x, y, 1); S2 = sum (K_s^-1 q) x
+                         * (K_s^T g), q = q_centre + x' (column 0 of H) + y' (column 1) */
+                        const float ks0 = pr.ks[0], ks1 = pr.ks[1], ks2 = pr.ks[2], ks3 = pr.ks[3];
+                        const float lam = fmaf(u0, px, fmaf(u1, py, u2));
+                        const float l0 = fmaf(lam, t0, fmaf(u0, x0, u1 * y0));
+                        const float l1 = fmaf(lam, t1, fmaf(u0, x1, u1 * y1));
+                        const float l2 = fmaf(lam, t2, fmaf(u0, x2, u1 * y2));
+                        S1x = ks0 * l0;
+                        S1y = ks1 * l1;
+                        S1z = fmaf(ks2, l0, fmaf(ks3, l1, l2));
+                        const float iks0 = 1.0f / ks0, iks1 = 1.0f / ks1;
+                        auto moment = [&](float q0, float q1, float q2, float s0, float s1, float s2) {
+                            const float p0 = fmaf(-ks2, q2, q0) * iks0, p1 = fmaf(-ks3, q2, q1) * iks1;
+                            const float e0 = ks0 * s0, e1 = ks1 * s1, e2 = fmaf(ks2, s0, fmaf(ks3, s1, s2));
+                            S2x += p1 * e2 - q2 * e1;
+                            S2y += q2 * e0 - p0 * e2;
+                            S2z += p0 * e1 - p1 * e0;
+                        };
+                        moment(fmaf(h[0], px, fmaf(h[1], py, h[2])), fmaf(h[3], px, fmaf(h[4], py, h[5])),
+                               fmaf(h[6], px, fmaf(h[7], py, h[8])), t0, t1, t2);
+                        moment(h[0], h[3], h[6], x0, x1, x2);
+                        moment(h[1], h[4], h[7], y0, y1, y2);
                     }
                 }
             }

@@ -68,3 +68,31 @@ def test_solve_near_borders_bit_exact(size, form):
     hyp, cost = s.read_hypotheses()
     assert_bit_equal(hyp, o.hyp, "hyp")
     assert_bit_equal(cost, o.cost, "cost")
+
+
+@pytest.mark.parametrize("size", [(12, 13), (33, 16), (64, 48)])
+def test_gradient_cost_at_borders_matches_plane_cost(size):
+    """The gradient kernel's forward cost of fronto-parallel planes (angles 0) is the sum of the plain
+    form's view costs: the same positions, so the same windows are lost (their cost, 2, is far from any
+    other by more than the tolerance), and the same FP32 sums but for the homography's composition
+    (1e-4 per source is the forward cost's tolerance elsewhere)."""
+    import torch
+
+    from luvas3d import grad
+
+    W, H = size
+    views = _views(W, H, 64.0)
+    rng = np.random.default_rng(W)
+    imgs = [rng.random((H, W)).astype(np.float32) for _ in views]
+    srcs = list(range(1, len(views)))
+    s = DenseStereo(W, H, views)
+    for i, im in enumerate(imgs):
+        s.set_image(i, im)
+    planes = np.zeros((H, W, 4), dtype=np.float32)
+    planes[..., 2] = -1.0
+    planes[..., 3] = rng.choice([0.125, 0.25, 0.5, 1.0, 2.0, 4.0], size=(H, W))
+    _, vc = s.plane_cost(0, SolveOptions(srcs, 0.05, 1e30), planes, view_costs=True)
+    pl = torch.zeros((H, W, 3), device="cuda")
+    pl[..., 0] = torch.from_numpy(planes[..., 3]).cuda()
+    got = grad.ncc_cost(s, 0, srcs, pl.contiguous()).cpu().numpy()
+    np.testing.assert_allclose(got, vc[..., :len(srcs)].sum(-1), rtol=0, atol=1e-4 * len(srcs))
