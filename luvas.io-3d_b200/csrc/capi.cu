@@ -1876,7 +1876,7 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
     if (e == cudaSuccess)
         e = l3d_launch_tsdf_brick_list(t->g, n, t->mask, sweep_flags(t), sweep_prefix(t), sweep_list(t),
                                        sweep_scratch(t), t->stream);
-    t->launches += 4 + (l3d_tsdf_super_flags(t->g, n) > 0 ? 1 : 0) + l3d_scan_launches(t->g.bricks + 1, false);
+    t->launches += 4 + (l3d_tsdf_super_flags(t->g, n) > 0 ? 1 : 0) + l3d_scan_launches(t->g.bricks + 1);
     if (e != cudaSuccess) return cuda_fail(e, "visibility launch");
     if (!tsdf_out && !weight_out) {
         e = l3d_launch_tsdf_many_list(t->g, t->views, n, t->coords, t->mask, t->depth_ptrs, t->priors,
@@ -2468,8 +2468,10 @@ struct DevBufs {
     }
 };
 
-int read_u32(const uint32_t* dev, uint32_t* host, cudaStream_t s) {
-    L3D_CUDA(cudaMemcpyAsync(host, dev, 4, cudaMemcpyDeviceToHost, s), "read count");
+/* `n` words of the device, after the work queued on `s`. */
+template <typename T>
+int read_words(const T* dev, T* host, cudaStream_t s, size_t n = 1) {
+    L3D_CUDA(cudaMemcpyAsync(host, dev, n * sizeof(T), cudaMemcpyDeviceToHost, s), "read count");
     L3D_CUDA(cudaStreamSynchronize(s), "synchronize");
     return L3D_OK;
 }
@@ -2484,21 +2486,28 @@ void mesh_free(l3d_mesh* m, cudaStream_t s = 0) {
     delete m;
 }
 
+/* The f32 bound with w < bound exactly when (double)w < min, for every f32 w. */
+float weight_bound(double min) {
+    const float f = (float)min;
+    return (double)f < min ? std::nextafterf(f, INFINITY) : f;
+}
+
 /* extractSurface (surface-nets.ts:47-174) + computeNormals (mesh.ts:9-31) of a volume view with
  * `bricks` bricks. */
 int extract_mesh(const L3dSdfView& v, long long bricks, cudaStream_t s, l3d_mesh** out) {
     const long long cells = bricks * 512;
     if (cells >= (1ll << 31)) return fail(L3D_EINVAL, "volume too large for surface extraction");
     DevBufs tmp(s);
-    uint32_t *flag, *base, *qcount, *qbase, *scratch, *total;
-    int32_t* cell_vertex;
-    L3D_CUDA(tmp.get(&flag, cells), "surface buffers");
-    L3D_CUDA(tmp.get(&base, cells), "surface buffers");
-    L3D_CUDA(tmp.get(&qcount, cells), "surface buffers");
-    L3D_CUDA(tmp.get(&qbase, cells), "surface buffers");
-    L3D_CUDA(tmp.get(&cell_vertex, cells), "surface buffers");
-    L3D_CUDA(tmp.get(&scratch, l3d_scan_scratch(std::max(cells, 1ll)) / 4 + 1), "scan scratch");
-    L3D_CUDA(tmp.get(&total, 2), "scan total");
+    L3dSurfaceBits bits;
+    unsigned long long *scratch, *total;
+    L3D_CUDA(tmp.get(&bits.obs, (size_t)bricks * 48), "surface buffers");
+    bits.neg = bits.obs + bricks * 16;
+    bits.flag = bits.neg + bricks * 16;
+    L3D_CUDA(tmp.get(&bits.rank, (size_t)bricks * 64), "surface buffers");
+    L3D_CUDA(tmp.get(&bits.count, (size_t)bricks * 2), "surface buffers");
+    bits.base = bits.count + bricks;
+    L3D_CUDA(tmp.get(&scratch, l3d_scan64_scratch(bricks) / 8 + 1), "scan scratch");
+    total = scratch + l3d_scan64_scratch(bricks) / 8;
     l3d_mesh* m = new (std::nothrow) l3d_mesh();
     if (!m) return fail(L3D_ENOMEM, "host allocation failed");
     auto bail = [&](int rc) {
@@ -2506,48 +2515,34 @@ int extract_mesh(const L3dSdfView& v, long long bricks, cudaStream_t s, l3d_mesh
         return rc;
     };
     cudaError_t e;
-    uint32_t nv = 0, nq = 0;
-    if ((e = l3d_launch_sn_flag(v, cells, flag, s)) != cudaSuccess ||
-        (e = l3d_scan_exclusive(flag, base, cells, scratch, total, s)) != cudaSuccess)
-        return bail(cuda_fail(e, "surface vertices"));
-    int rc = read_u32(total, &nv, s);
+    if ((e = l3d_launch_sn_bits(v, bricks, bits, s)) != cudaSuccess ||
+        (e = l3d_scan64_exclusive(bits.count, bits.base, bricks, scratch, total, s)) != cudaSuccess)
+        return bail(cuda_fail(e, "surface counts"));
+    unsigned long long counts = 0;
+    int rc = read_words(total, &counts, s);
     if (rc) return bail(rc);
-    double* pos_d;
-    if ((e = tmp.get(&pos_d, (size_t)nv * 3)) != cudaSuccess ||
-        (e = pool_alloc((void**)&m->pos, std::max<size_t>(nv, 1) * 12, s)) != cudaSuccess ||
-        (e = pool_alloc((void**)&m->nrm, std::max<size_t>(nv, 1) * 12, s)) != cudaSuccess)
-        return bail(cuda_fail(e, "vertex buffers"));
-    if ((e = l3d_launch_sn_vertex(v, cells, flag, base, cell_vertex, pos_d, m->pos, s)) != cudaSuccess ||
-        (e = l3d_launch_sn_count(v, cells, cell_vertex, qcount, s)) != cudaSuccess ||
-        (e = l3d_scan_exclusive(qcount, qbase, cells, scratch, total, s)) != cudaSuccess)
-        return bail(cuda_fail(e, "surface quads"));
-    if ((rc = read_u32(total, &nq, s))) return bail(rc);
+    const uint32_t nv = (uint32_t)counts, nq = (uint32_t)(counts >> 32);
     const long long faces = 2ll * nq;
-    if ((e = pool_alloc((void**)&m->idx, std::max<long long>(faces * 3, 1) * 4, s)) != cudaSuccess)
-        return bail(cuda_fail(e, "index buffer"));
-    if ((e = l3d_launch_sn_emit(v, cells, cell_vertex, qcount, qbase, pos_d, m->idx, s)) != cudaSuccess)
-        return bail(cuda_fail(e, "surface triangles"));
-    /* normals: faces gathered per vertex in face order */
-    double* fn;
-    uint32_t *degree, *start, *cursor, *lists;
-    if ((e = tmp.get(&fn, (size_t)faces * 3)) != cudaSuccess || (e = tmp.get(&degree, nv)) != cudaSuccess ||
-        (e = tmp.get(&start, nv)) != cudaSuccess || (e = tmp.get(&cursor, nv)) != cudaSuccess ||
-        (e = tmp.get(&lists, (size_t)faces * 3)) != cudaSuccess)
-        return bail(cuda_fail(e, "normal buffers"));
-    uint32_t* nscratch;
-    if ((e = tmp.get(&nscratch, l3d_scan_scratch(std::max<long long>(nv, 1)) / 4 + 1)) != cudaSuccess)
-        return bail(cuda_fail(e, "scan scratch"));
-    if ((e = cudaMemsetAsync(degree, 0, std::max<size_t>(nv, 1) * 4, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(cursor, 0, std::max<size_t>(nv, 1) * 4, s)) != cudaSuccess ||
-        (e = l3d_launch_face_normals(m->pos, m->idx, faces, fn, degree, s)) != cudaSuccess ||
+    double *pos_d, *fn;
+    uint32_t *degree, *start, *lists, *nscratch;
+    if ((e = tmp.get(&pos_d, (size_t)nv * 3 + (size_t)faces * 3)) != cudaSuccess ||
+        (e = tmp.get(&degree, (size_t)nv * 2 + (size_t)faces * 3 + l3d_scan_scratch(nv) / 4)) != cudaSuccess ||
+        (e = pool_alloc((void**)&m->pos, std::max<size_t>(nv, 1) * 12, s)) != cudaSuccess ||
+        (e = pool_alloc((void**)&m->nrm, std::max<size_t>(nv, 1) * 12, s)) != cudaSuccess ||
+        (e = pool_alloc((void**)&m->idx, std::max<long long>(faces * 3, 1) * 4, s)) != cudaSuccess)
+        return bail(cuda_fail(e, "mesh buffers"));
+    fn = pos_d + (size_t)nv * 3;
+    start = degree + nv;
+    lists = start + nv;
+    nscratch = lists + (size_t)faces * 3;
+    if ((e = l3d_launch_sn_emit(v, bricks, bits, pos_d, m->pos, m->idx, fn, degree, s)) != cudaSuccess ||
         (e = l3d_scan_exclusive(degree, start, nv, nscratch, nullptr, s)) != cudaSuccess ||
-        (e = l3d_launch_face_lists(m->idx, faces, start, cursor, lists, s)) != cudaSuccess ||
-        (e = l3d_launch_vertex_normals(nv, start, degree, lists, fn, m->nrm, s)) != cudaSuccess ||
+        (e = l3d_launch_vertex_normals(m->idx, faces, nv, start, degree, lists, fn, m->nrm, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return bail(cuda_fail(e, "vertex normals"));
+        return bail(cuda_fail(e, "surface vertices, triangles and normals"));
     m->nv = nv;
     m->ni = faces * 3;
-    m->launches = 13;
+    m->launches = 7 + l3d_scan_launches(bricks) + l3d_scan_launches(nv);
     *out = m;
     return L3D_OK;
 }
@@ -2576,7 +2571,7 @@ int l3d_tsdf_extract_surface(l3d_tsdf* t, double min_weight, l3d_mesh** out) {
     v.q8 = t->q8;
     for (int i = 0; i < 3; i++) v.origin[i] = t->g.origin_d[i];
     v.voxel = t->g.voxel_d;
-    v.min_weight = min_weight;
+    v.min_weight_f = weight_bound(min_weight);
     DevBufs tmp(t->stream);
     long long bricks;
     if (t->g.dense) {
@@ -2655,7 +2650,7 @@ int l3d_extract_surface(const l3d_sdf_bricks* vol, double min_weight, l3d_mesh**
         v.origin[i] = vol->origin[i];
     }
     v.voxel = vol->voxel;
-    v.min_weight = min_weight;
+    v.min_weight_f = weight_bound(min_weight);
     return extract_mesh(v, vol->bricks, s, out);
 }
 
@@ -2689,60 +2684,46 @@ int l3d_mesh_remove_small_components(const l3d_mesh* m, double fraction, int32_t
         }
     } guard{s};
     DevBufs tmp(s);
-    uint32_t *label, *comp, *kept, *first, *face_base, *marks, *rank, *scratch, *total;
-    int* changed;
-    L3D_CUDA(tmp.get(&label, nv), "component buffers");
-    L3D_CUDA(tmp.get(&comp, nv), "component buffers");
-    L3D_CUDA(tmp.get(&kept, faces), "component buffers");
-    L3D_CUDA(tmp.get(&first, nv), "component buffers");
-    L3D_CUDA(tmp.get(&face_base, faces), "component buffers");
-    L3D_CUDA(tmp.get(&marks, faces * 3), "component buffers");
-    L3D_CUDA(tmp.get(&rank, faces * 3), "component buffers");
-    L3D_CUDA(tmp.get(&scratch, l3d_scan_scratch(std::max(faces * 3, 1ll)) / 4 + 1), "scan scratch");
-    L3D_CUDA(tmp.get(&total, 2), "scan total");
-    L3D_CUDA(tmp.get(&changed, 1), "flag");
-    L3D_CUDA(l3d_launch_cc_init(nv, label, s), "component labels");
-    /* rounds in batches of 8 between host checks: once the labels have settled a round changes
-     * nothing, so the extra rounds of the last batch leave the result as it is */
-    int rounds = 0;
-    for (;;) {
-        if (rounds >= 256) return fail(L3D_ECUDA, "connected components did not settle in 256 rounds");
-        int h = 0;
-        L3D_CUDA(cudaMemsetAsync(changed, 0, sizeof(int), s), "flag clear");
-        for (int k = 0; k < 8; k++, rounds++)
-            L3D_CUDA(l3d_launch_cc_round(m->idx, faces, nv, label, changed, s), "component round");
-        L3D_CUDA(cudaMemcpyAsync(&h, changed, sizeof(int), cudaMemcpyDeviceToHost, s), "flag read");
-        L3D_CUDA(cudaStreamSynchronize(s), "synchronize");
-        if (!h) break;
-    }
+    uint32_t *label, *comp, *first;
+    unsigned long long *pack, *base, *scratch, *total;
+    int* err;
+    L3D_CUDA(tmp.get(&label, (size_t)nv * 3), "component buffers");
+    comp = label + nv;
+    first = comp + nv;
+    L3D_CUDA(tmp.get(&pack, (size_t)faces * 2), "component buffers");
+    base = pack + faces;
+    /* the scan's scratch, its total and the labels' error flag */
+    const size_t words = l3d_scan64_scratch(faces) / 8;
+    L3D_CUDA(tmp.get(&scratch, words + 2), "scan scratch");
+    total = scratch + words;
+    err = (int*)(total + 1);
     const double limit = std::max((double)min_faces, (double)faces * fraction);
-    uint32_t kf = 0, kv = 0;
+    L3D_CUDA(cudaMemsetAsync(total, 0, 16, s), "clear");
+    L3D_CUDA(l3d_launch_cc_labels(m->idx, faces, nv, label, err, s), "component labels");
     L3D_CUDA(cudaMemsetAsync(comp, 0, std::max<size_t>(nv, 1) * 4, s), "clear");
     L3D_CUDA(cudaMemsetAsync(first, 0xff, std::max<size_t>(nv, 1) * 4, s), "clear");
-    L3D_CUDA(cudaMemsetAsync(marks, 0, std::max<size_t>(faces * 3, 1) * 4, s), "clear");
-    L3D_CUDA(l3d_launch_cc_count(m->idx, faces, label, comp, s), "component sizes");
-    L3D_CUDA(l3d_launch_cc_keep(m->idx, faces, label, comp, limit, kept, first, s), "kept faces");
-    L3D_CUDA(l3d_scan_exclusive(kept, face_base, faces, scratch, total, s), "face scan");
-    int rc = read_u32(total, &kf, s);
+    L3D_CUDA(l3d_launch_cc_keep(m->idx, faces, label, comp, limit, first, pack, s), "kept faces");
+    L3D_CUDA(l3d_scan64_exclusive(pack, base, faces, scratch, total, s), "face scan");
+    unsigned long long found[2] = {0, 0};
+    int rc = read_words(total, found, s, 2);
     if (rc) return rc;
-    L3D_CUDA(l3d_launch_cc_first_marks(nv, first, marks, s), "vertex order");
-    L3D_CUDA(l3d_scan_exclusive(marks, rank, faces * 3, scratch, total, s), "vertex scan");
-    if ((rc = read_u32(total, &kv, s))) return rc;
+    if ((uint32_t)found[1]) return fail(L3D_ECUDA, "connected components did not settle");
+    const uint32_t kf = (uint32_t)found[0], kv = (uint32_t)(found[0] >> 32);
     l3d_mesh* r = new (std::nothrow) l3d_mesh();
     if (!r) return fail(L3D_ENOMEM, "host allocation failed");
     cudaError_t e;
     if ((e = pool_alloc((void**)&r->pos, std::max<size_t>(kv, 1) * 12, s)) != cudaSuccess ||
         (e = pool_alloc((void**)&r->nrm, std::max<size_t>(kv, 1) * 12, s)) != cudaSuccess ||
         (e = pool_alloc((void**)&r->idx, std::max<size_t>(kf, 1) * 12, s)) != cudaSuccess ||
-        (e = l3d_launch_cc_emit(m->idx, faces, kept, face_base, first, rank, m->pos, m->nrm, r->idx,
-                                r->pos, r->nrm, s)) != cudaSuccess ||
+        (e = l3d_launch_cc_emit(m->idx, faces, pack, base, first, m->pos, m->nrm, r->idx, r->pos, r->nrm,
+                                s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess) {
         mesh_free(r, s);
         return cuda_fail(e, "component output");
     }
     r->nv = kv;
     r->ni = 3ll * kf;
-    r->launches = 2ll * rounds + 9;
+    r->launches = 7 + l3d_scan_launches(faces);
     *out = r;
     return L3D_OK;
 }
@@ -2798,7 +2779,7 @@ int l3d_brick_grid_build(const double origin[3], double voxel, const double exte
     L3D_CUDA(l3d_launch_grid_widen(marks, cells, flags, s), "mark");
     L3D_CUDA(l3d_scan_exclusive(flags, base, cells, scratch, total, s), "brick scan");
     uint32_t c = 0;
-    int rc = read_u32(total, &c, s);
+    int rc = read_words(total, &c, s);
     if (rc) return rc;
     *count = (int32_t)c;
     L3D_CUDA(tmp.get(&dcoords, (size_t)c * 4), "coords buffer");

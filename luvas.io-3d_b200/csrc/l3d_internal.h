@@ -352,13 +352,16 @@ cudaError_t l3d_launch_cloud_emit_sorted(const L3dCloudTable& t, unsigned total,
 
 /* ---- prefix sums (scan.cu) ---- */
 
-/* Bytes of scratch l3d_scan_exclusive needs for n elements. */
+/* Bytes of scratch l3d_scan_exclusive / l3d_scan64_exclusive need for n elements. */
 size_t l3d_scan_scratch(long long n);
-/* Kernel launches l3d_scan_exclusive makes for n elements (with or without `total`). */
-int l3d_scan_launches(long long n, bool total);
+size_t l3d_scan64_scratch(long long n);
+/* Kernel launches of either scan for n elements. */
+int l3d_scan_launches(long long n);
 /* out[i] = in[0] + ... + in[i-1] (in == out allowed); *total (device, may be NULL) = the sum. */
 cudaError_t l3d_scan_exclusive(const uint32_t* in, uint32_t* out, long long n, uint32_t* scratch,
                                uint32_t* total, cudaStream_t stream);
+cudaError_t l3d_scan64_exclusive(const unsigned long long* in, unsigned long long* out, long long n,
+                                 unsigned long long* scratch, unsigned long long* total, cudaStream_t stream);
 
 /* ---- surface extraction (mesh.cu) ---- */
 
@@ -375,7 +378,7 @@ struct L3dSdfView {
     int q8;
     double origin[3];
     double voxel;
-    double min_weight;
+    float min_weight_f;        /* the smallest f32 that is at least the minimum weight */
 };
 
 struct L3dBrickGrid {
@@ -384,33 +387,36 @@ struct L3dBrickGrid {
     int dims[3];
 };
 
-cudaError_t l3d_launch_sn_flag(const L3dSdfView& v, long long cells, uint32_t* flag, cudaStream_t s);
-cudaError_t l3d_launch_sn_vertex(const L3dSdfView& v, long long cells, const uint32_t* flag,
-                                 const uint32_t* base, int32_t* cell_vertex, double* pos_d,
-                                 float* pos_f, cudaStream_t s);
-cudaError_t l3d_launch_sn_count(const L3dSdfView& v, long long cells, const int32_t* cell_vertex,
-                                uint32_t* qcount, cudaStream_t s);
-cudaError_t l3d_launch_sn_emit(const L3dSdfView& v, long long cells, const int32_t* cell_vertex,
-                               const uint32_t* qcount, const uint32_t* qbase, const double* pos_d,
-                               uint32_t* indices, cudaStream_t s);
-cudaError_t l3d_launch_face_normals(const float* pos, const uint32_t* idx, long long faces, double* fn,
-                                    uint32_t* degree, cudaStream_t s);
-cudaError_t l3d_launch_face_lists(const uint32_t* idx, long long faces, const uint32_t* start,
-                                  uint32_t* cursor, uint32_t* lists, cudaStream_t s);
-cudaError_t l3d_launch_vertex_normals(long long vertices, const uint32_t* start, const uint32_t* degree,
-                                      uint32_t* lists, const double* fn, float* nrm, cudaStream_t s);
-cudaError_t l3d_launch_cc_init(long long vertices, uint32_t* label, cudaStream_t s);
-cudaError_t l3d_launch_cc_round(const uint32_t* idx, long long faces, long long vertices, uint32_t* label,
-                                int* changed, cudaStream_t s);
-cudaError_t l3d_launch_cc_count(const uint32_t* idx, long long faces, const uint32_t* label,
-                                uint32_t* comp_faces, cudaStream_t s);
-cudaError_t l3d_launch_cc_keep(const uint32_t* idx, long long faces, const uint32_t* label,
-                               const uint32_t* comp_faces, double limit, uint32_t* kept,
-                               uint32_t* first, cudaStream_t s);
-cudaError_t l3d_launch_cc_first_marks(long long vertices, const uint32_t* first, uint32_t* marks,
+/* Per brick, one bit per voxel or cell (bit x of byte y + 8 z): `obs` observed voxels, `neg` negative
+ * ones among them, `flag` cells with a vertex; rank[b * 64 + row]: flagged cells in the rows before
+ * (written for bricks that have any); count[b] and base[b]: vertices (low 32 bits) and quads (high). */
+struct L3dSurfaceBits {
+    uint32_t *obs, *neg, *flag;        /* 16 words per brick */
+    uint16_t* rank;                    /* 64 per brick */
+    unsigned long long *count, *base;  /* 1 per brick */
+};
+/* bits of every voxel, flags and vertex counts of every brick, quad counts: three launches */
+cudaError_t l3d_launch_sn_bits(const L3dSdfView& v, long long bricks, const L3dSurfaceBits& t, cudaStream_t s);
+/* vertices and triangles behind base[], the triangles' normals fn (3 doubles each) and the number of
+ * triangles at each vertex: two launches */
+cudaError_t l3d_launch_sn_emit(const L3dSdfView& v, long long bricks, const L3dSurfaceBits& t, double* pos_d,
+                               float* pos_f, uint32_t* indices, double* fn, uint32_t* degree, cudaStream_t s);
+/* vertex normals from the triangles' (start: exclusive prefix sums of degree, overwritten; lists: 3 per
+ * face): two launches */
+cudaError_t l3d_launch_vertex_normals(const uint32_t* idx, long long faces, long long vertices, uint32_t* start,
+                                      const uint32_t* degree, uint32_t* lists, const double* fn, float* nrm,
                                       cudaStream_t s);
-cudaError_t l3d_launch_cc_emit(const uint32_t* idx, long long faces, const uint32_t* kept,
-                               const uint32_t* face_base, const uint32_t* first, const uint32_t* rank,
+/* connected components: label[v] = one vertex of v's component, the same for all of them; *err set when a
+ * chain of labels was longer than any can be (three launches) */
+cudaError_t l3d_launch_cc_labels(const uint32_t* idx, long long faces, long long vertices, uint32_t* label,
+                                 int* err, cudaStream_t s);
+/* comp_faces[label] (zeroed), first[v] (all ones) = first corner of a kept face that uses v, pack[f] =
+ * kept (low 32 bits) and the number of f's corners that are their vertex's first (high): three launches */
+cudaError_t l3d_launch_cc_keep(const uint32_t* idx, long long faces, const uint32_t* label,
+                               uint32_t* comp_faces, double limit, uint32_t* first,
+                               unsigned long long* pack, cudaStream_t s);
+cudaError_t l3d_launch_cc_emit(const uint32_t* idx, long long faces, const unsigned long long* pack,
+                               const unsigned long long* base, const uint32_t* first,
                                const float* pos, const float* nrm, uint32_t* out_idx, float* out_pos,
                                float* out_nrm, cudaStream_t s);
 cudaError_t l3d_launch_grid_mark(const float* pts, long long n, const L3dBrickGrid& g, double radius,
