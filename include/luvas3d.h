@@ -528,9 +528,11 @@ int l3d_measure_fetch_rate(int32_t dtype, int32_t checker, int32_t mode, double*
  * library's own on each device, which keeps up to 16 GB of freed memory mapped for the next
  * call.  l3d_memory_trim waits for the current device's queued work, then hands the pool's
  * unused memory back to the driver until at most keep_bytes stay reserved (0 releases all of
- * it); memory held by live handles stays.  It replaces what GPUBuffer.destroy() does for the
- * reference at once (fusion/tsdf-volume.ts:279-290, mvs/dense-stereo.ts:357-370): a caller
- * that shares the device with another allocator calls it after destroying handles. */
+ * it); memory held by live handles stays.  It also destroys the few streams and pinned buffers
+ * that the library keeps between mesh, cloud and brick-grid calls.  It replaces what
+ * GPUBuffer.destroy() does for the reference at once (fusion/tsdf-volume.ts:279-290,
+ * mvs/dense-stereo.ts:357-370): a caller that shares the device with another allocator calls it
+ * after destroying handles. */
 int l3d_memory_trim(int64_t keep_bytes);
 
 /* The current device pool's reserved bytes (mapped: in use plus freed and kept) and the part

@@ -89,9 +89,9 @@ class PointAccumulator:
         """cloud(minSupport) (point-accumulator.ts:114-143), ordered by cell.  One read into
         buffers sized for every occupied cell, trimmed to the points returned."""
         k = self.size
-        out = PointCloud(np.zeros((k, 3), np.float32), np.zeros((k, 3), np.float32),
-                         np.zeros((k, 3), np.uint8), np.zeros(k, np.uint16),
-                         np.zeros((k, 3), np.int32))
+        out = PointCloud(np.empty((k, 3), np.float32), np.empty((k, 3), np.float32),
+                         np.empty((k, 3), np.uint8), np.empty(k, np.uint16),
+                         np.empty((k, 3), np.int32))
         n = C.c_int64()
         _lib.check(self._lib.l3d_cloud_read(self._h(), int(min_support), k, C.byref(n),
                                             _lib.ptr(out.positions), _lib.ptr(out.normals),

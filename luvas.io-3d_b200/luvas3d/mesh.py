@@ -36,7 +36,7 @@ class DeviceMesh:
 
     def read(self) -> Mesh:
         nv, ni = self.counts
-        m = Mesh(np.zeros((nv, 3), np.float32), np.zeros((nv, 3), np.float32), np.zeros(ni, np.uint32))
+        m = Mesh(np.empty((nv, 3), np.float32), np.empty((nv, 3), np.float32), np.empty(ni, np.uint32))
         _lib.check(self._lib.l3d_mesh_read(self._handle, _lib.ptr(m.positions), _lib.ptr(m.normals),
                                            _lib.ptr(m.indices)))
         return m

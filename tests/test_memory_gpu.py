@@ -44,3 +44,47 @@ def test_trim_releases_destroyed_handles_memory_and_keeps_live_handles():
     live.add_points(samples(1000, 3))
     assert live.size > first.positions.shape[0]
     live.destroy()
+
+
+def test_reads_of_every_size_survive_trimming_and_threads():
+    """Read-backs go through two kept pinned buffers of 1 MB: clouds smaller than one, around one and
+    two, and of several, read from several threads at once, before and after the buffers are given
+    back, equal the samples that went in."""
+    import threading
+
+    def check(n, seed):
+        rng = np.random.default_rng(seed)
+        cell = 0.01
+        ids = rng.choice(200 ** 3, n, replace=False)
+        at = np.stack([ids % 200, ids // 200 % 200, ids // 40000], 1)
+        s = samples(n, seed)
+        s[:, :3] = (at + 0.5) * cell
+        s[:, 6:] = at % 251
+        acc = PointAccumulator(cell)
+        acc.add_points(s)
+        c = acc.cloud()
+        acc.destroy()
+        order = np.lexsort((at[:, 0], at[:, 1], at[:, 2]))
+        np.testing.assert_array_equal(c.cells, at[order])
+        np.testing.assert_array_equal(c.positions, s[order, :3].astype(np.float32))
+        np.testing.assert_array_equal(c.colors, (at[order] % 251).astype(np.uint8))
+        assert (c.support == 1).all()
+
+    failed = []
+
+    def work(n, seed):
+        try:
+            check(n, seed)
+        except BaseException as e:  # noqa: BLE001
+            failed.append((n, e))
+
+    for _ in range(2):
+        for n in (1, 25575, 25576, 51150, 51151, 300000):  # 41 bytes a point
+            check(n, n)
+        threads = [threading.Thread(target=work, args=(30000 + 9000 * i, i)) for i in range(7)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not failed, failed
+        trim_memory(0)
