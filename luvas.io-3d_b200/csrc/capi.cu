@@ -2260,8 +2260,7 @@ void l3d_tsdf_destroy(l3d_tsdf* t) {
 struct l3d_cloud {
     double cell = 0.0;
     L3dCloudTable t{};
-    unsigned* counters = nullptr;     /* [0] used slots, [1] emitted points */
-    int* err = nullptr;
+    L3dCloudState* state = nullptr;
     cudaStream_t stream = nullptr;
     Courier* courier = nullptr;       /* the cloud's own stream, when it was given none */
     cudaEvent_t done = nullptr;
@@ -2306,17 +2305,17 @@ int alloc_table(l3d_cloud* c, int capacity, L3dCloudTable* out) {
 }
 
 /* Waits for the queued work and reports a device-side error of the table. */
-int cloud_state(l3d_cloud* c, unsigned* used) {
-    unsigned h[2];
-    int err = 0;
-    L3D_CUDA(cudaMemcpyAsync(h, c->counters, sizeof(h), cudaMemcpyDeviceToHost, c->stream), "read counters");
-    L3D_CUDA(cudaMemcpyAsync(&err, c->err, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "read error flag");
+int cloud_state(l3d_cloud* c, unsigned* used, L3dCloudState* all = nullptr) {
+    L3dCloudState h;
+    L3D_CUDA(cudaMemcpyAsync(&h, c->state, sizeof(h), cudaMemcpyDeviceToHost, c->stream), "read counters");
     L3D_CUDA(cudaStreamSynchronize(c->stream), "synchronize");
+    const int err = h.err;
     if (err & L3D_CLOUD_ERR_RANGE)
         return fail(L3D_EINVAL, "a point lies more than 2^20 cells from the origin (cell %g m)", c->cell);
     if (err & L3D_CLOUD_ERR_FULL) return fail(L3D_ECUDA, "point table overflow");
-    if (used) *used = h[0];
-    c->used_bound = h[0];
+    if (used) *used = h.used;
+    if (all) *all = h;
+    c->used_bound = h.used;
     return L3D_OK;
 }
 
@@ -2325,8 +2324,8 @@ int cloud_rebuild(l3d_cloud* c, int capacity, double cell) {
     L3dCloudTable nt;
     int rc = alloc_table(c, capacity, &nt);
     if (rc) return rc;
-    L3D_CUDA(cudaMemsetAsync(c->counters, 0, sizeof(unsigned), c->stream), "reset counter");
-    cudaError_t e = l3d_launch_cloud_rebin(c->t, nt, cell, c->counters, c->err, c->stream);
+    L3D_CUDA(cudaMemsetAsync(&c->state->used, 0, sizeof(unsigned), c->stream), "reset counter");
+    cudaError_t e = l3d_launch_cloud_rebin(c->t, nt, cell, &c->state->used, &c->state->err, c->stream);
     c->launches++;
     if (e != cudaSuccess) {
         free_table(nt, c->stream);
@@ -2357,6 +2356,24 @@ int cloud_reserve(l3d_cloud* c, long long extra) {
     c->used_bound = (long long)used + extra;
     return L3D_OK;
 }
+
+/* Scratch buffers allocated and freed in the order of stream `s` (no device-wide wait), freed
+ * when the holder goes out of scope. */
+struct DevBufs {
+    cudaStream_t s;
+    std::vector<void*> ptrs;
+    explicit DevBufs(cudaStream_t stream) : s(stream) {}
+    ~DevBufs() {
+        for (void* p : ptrs) cudaFreeAsync(p, s);
+    }
+    template <typename T>
+    cudaError_t get(T** p, size_t count) {
+        *p = nullptr;
+        cudaError_t e = pool_alloc((void**)p, std::max<size_t>(count, 1) * sizeof(T), s);
+        if (e == cudaSuccess) ptrs.push_back(*p);
+        return e;
+    }
+};
 
 template <typename T>
 int ensure_upload(T** p, size_t* cap, size_t n, cudaStream_t stream, const char* what) {
@@ -2393,11 +2410,9 @@ int l3d_cloud_create(double cell, void* stream, l3d_cloud** out) {
     }
     if ((e = cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming)) != cudaSuccess)
         return cleanup(cuda_fail(e, "event creation"));
-    if ((e = pool_alloc((void**)&c->counters, 2 * sizeof(unsigned), c->stream)) != cudaSuccess ||
-        (e = pool_alloc((void**)&c->err, sizeof(int), c->stream)) != cudaSuccess)
+    if ((e = pool_alloc((void**)&c->state, sizeof(L3dCloudState), c->stream)) != cudaSuccess)
         return cleanup(cuda_fail(e, "counter allocation"));
-    if ((e = cudaMemsetAsync(c->counters, 0, 2 * sizeof(unsigned), c->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(c->err, 0, sizeof(int), c->stream)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(c->state, 0, sizeof(L3dCloudState), c->stream)) != cudaSuccess)
         return cleanup(cuda_fail(e, "counter clear"));
     int rc = alloc_table(c, 1 << 16, &c->t);
     if (rc) return cleanup(rc);
@@ -2444,8 +2459,10 @@ int l3d_cloud_add(l3d_cloud* c, const l3d_stereo* src, const uint32_t* packed, i
     for (int i = 0; i < 3; i++) v.t[i] = view->pose.t[i];
     v.tw = thumb_w;
     v.th = thumb_h;
-    cudaError_t e = l3d_launch_cloud_add_map(c->t, c->cell, map, W, H, v, c->thumb, c->counters,
-                                             c->err, c->stream);
+    v.sx = (double)thumb_w / W;
+    v.sy = (double)thumb_h / H;
+    cudaError_t e = l3d_launch_cloud_add_map(c->t, c->cell, map, W, H, v, c->thumb, &c->state->used,
+                                             &c->state->err, c->stream);
     c->launches++;
     if (e != cudaSuccess) return cuda_fail(e, "point add launch");
     if (src) {
@@ -2465,7 +2482,8 @@ int l3d_cloud_add_points(l3d_cloud* c, int64_t n, const double* samples) {
     if ((rc = ensure_upload(&c->pts, &c->pts_cap, (size_t)n * 9, c->stream, "sample buffer"))) return rc;
     L3D_CUDA(cudaMemcpyAsync(c->pts, samples, (size_t)n * 9 * 8, cudaMemcpyHostToDevice, c->stream),
              "sample upload");
-    cudaError_t e = l3d_launch_cloud_add_points(c->t, c->cell, c->pts, n, c->counters, c->err, c->stream);
+    cudaError_t e = l3d_launch_cloud_add_points(c->t, c->cell, c->pts, n, &c->state->used, &c->state->err,
+                                                c->stream);
     c->launches++;
     if (e != cudaSuccess) return cuda_fail(e, "point add launch");
     return L3D_OK;
@@ -2498,77 +2516,66 @@ int l3d_cloud_read(l3d_cloud* c, int32_t min_support, int64_t capacity, int64_t*
                    float* positions, float* normals, uint8_t* colors, uint16_t* support,
                    int32_t* cells) {
     if (!c || !count) return fail(L3D_EINVAL, "NULL handle or count");
-    unsigned used = 0;
-    int rc = cloud_state(c, &used);
-    if (rc) return rc;
-    const unsigned sort_n = l3d_cloud_sort_length(std::max<unsigned>(used, 1u));
-    unsigned long long* dkey = nullptr;
-    uint32_t* dslot = nullptr;
-    float* dpos = nullptr;
-    float* dnrm = nullptr;
-    uint8_t* dcol = nullptr;
-    uint16_t* dsup = nullptr;
-    int32_t* dcell = nullptr;
-    cudaError_t e;
-    auto cleanup = [&]() {
-        for (void* q : {(void*)dkey, (void*)dslot, (void*)dpos, (void*)dnrm, (void*)dcol, (void*)dsup,
-                        (void*)dcell})
-            if (q) cudaFreeAsync(q, c->stream);
-    };
-    if ((e = pool_alloc((void**)&dkey, (size_t)sort_n * 8, c->stream)) != cudaSuccess ||
-        (e = pool_alloc((void**)&dslot, (size_t)sort_n * 4, c->stream)) != cudaSuccess) {
-        cleanup();
-        return cuda_fail(e, "read buffers");
-    }
-    unsigned total = 0;
-    if ((e = cudaMemsetAsync(c->counters + 1, 0, sizeof(unsigned), c->stream)) != cudaSuccess ||
-        (e = l3d_launch_cloud_emit_keys(c->t, (unsigned)std::max(min_support, 0), c->counters + 1, dkey,
-                                        dslot, c->stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&total, c->counters + 1, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                             c->stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(c->stream)) != cudaSuccess) {
-        cleanup();
-        return cuda_fail(e, "point read");
-    }
+    /* the state and, queued before it is read, the number and box of the points to return */
+    const unsigned least = (unsigned)std::max(min_support, 0);
+    L3D_CUDA(cudaMemsetAsync(&c->state->total, 0, 4 * sizeof(unsigned), c->stream), "reset counter");
+    L3D_CUDA(cudaMemsetAsync(c->state->lo, 0xff, 3 * sizeof(unsigned), c->stream), "reset counter");
+    L3D_CUDA(l3d_launch_cloud_box(c->t, least, c->state, c->stream), "point count");
     c->launches++;
+    L3dCloudState h;
+    int rc = cloud_state(c, nullptr, &h);
+    if (rc) return rc;
+    const unsigned total = h.total;
     *count = total;
-    if (!positions && !normals && !colors && !support && !cells) {
-        cleanup();
-        return L3D_OK;
-    }
-    if (capacity < (int64_t)total) {
-        cleanup();
+    if (!positions && !normals && !colors && !support && !cells) return L3D_OK;
+    if (capacity < (int64_t)total)
         return fail(L3D_EINVAL, "output holds %lld points, the cloud has %u", (long long)capacity, total);
+    if (!total) return L3D_OK;
+    DevBufs tmp(c->stream);
+    /* cells in ascending packed order (z, then y, then x; keys are distinct), ordered and gathered on
+     * the device, then copied into the caller's arrays */
+    L3dCloudOut d;
+    cudaError_t e;
+    if ((e = tmp.get(&d.pos, (size_t)total * 6)) != cudaSuccess || (e = tmp.get(&d.cells, (size_t)total * 3)) != cudaSuccess ||
+        (e = tmp.get(&d.support, total)) != cudaSuccess || (e = tmp.get(&d.col, (size_t)total * 3)) != cudaSuccess)
+        return cuda_fail(e, "read buffers");
+    d.nrm = d.pos + (size_t)total * 3;
+    L3dCloudBox box;
+    for (int k = 0; k < 3; k++) {
+        box.lo[k] = h.lo[k];
+        box.dims[k] = h.hi[k] - h.lo[k] + 1u;
     }
-    /* cells in ascending packed order (z, then y, then x; keys are distinct), sorted and
-     * gathered on the device, then copied straight into the caller's arrays */
-    const size_t m = std::max<unsigned>(total, 1u);
-    if ((e = pool_alloc((void**)&dpos, m * 12, c->stream)) != cudaSuccess ||
-        (e = pool_alloc((void**)&dnrm, m * 12, c->stream)) != cudaSuccess ||
-        (e = pool_alloc((void**)&dcol, m * 3, c->stream)) != cudaSuccess ||
-        (e = pool_alloc((void**)&dsup, m * 2, c->stream)) != cudaSuccess ||
-        (e = pool_alloc((void**)&dcell, m * 12, c->stream)) != cudaSuccess ||
-        (e = l3d_launch_cloud_sort(dkey, dslot, total, sort_n, &c->launches, c->stream)) != cudaSuccess ||
-        (e = l3d_launch_cloud_emit_sorted(c->t, total, dkey, dslot, dpos, dnrm, dcol, dsup, dcell,
-                                          c->stream)) != cudaSuccess) {
-        cleanup();
-        return cuda_fail(e, "point ordering");
+    if (const long long groups = l3d_cloud_box_groups(box, total)) {
+        uint32_t *bits, *before;
+        if ((e = tmp.get(&bits, (size_t)groups * 8)) != cudaSuccess ||
+            (e = tmp.get(&before, (size_t)groups + l3d_scan_scratch(groups) / 4)) != cudaSuccess ||
+            (e = l3d_launch_cloud_emit_placed(c->t, least, box, groups, bits, before, before + groups, d,
+                                              c->stream)) != cudaSuccess)
+            return cuda_fail(e, "point ordering");
+        c->launches += 3 + l3d_scan_launches(groups);
+    } else {
+        const unsigned sort_n = l3d_cloud_sort_length(total);
+        unsigned long long* keys;
+        uint32_t* slots;
+        if ((e = tmp.get(&keys, sort_n)) != cudaSuccess || (e = tmp.get(&slots, sort_n)) != cudaSuccess ||
+            (e = cudaMemsetAsync(&c->state->total, 0, sizeof(unsigned), c->stream)) != cudaSuccess ||
+            (e = l3d_launch_cloud_emit_keys(c->t, least, &c->state->total, keys, slots, c->stream)) != cudaSuccess ||
+            (e = l3d_launch_cloud_sort(keys, slots, total, sort_n, &c->launches, c->stream)) != cudaSuccess ||
+            (e = l3d_launch_cloud_emit_sorted(c->t, total, keys, slots, d, c->stream)) != cudaSuccess)
+            return cuda_fail(e, "point ordering");
+        c->launches += 2;
     }
-    c->launches += total ? 1 : 0;
-    const HostOut outs[] = {{positions, dpos, (size_t)total * 12}, {normals, dnrm, (size_t)total * 12},
-                            {colors, dcol, (size_t)total * 3}, {support, dsup, (size_t)total * 2},
-                            {cells, dcell, (size_t)total * 12}};
+    const HostOut outs[] = {{positions, d.pos, (size_t)total * 12}, {normals, d.nrm, (size_t)total * 12},
+                            {colors, d.col, (size_t)total * 3}, {support, d.support, (size_t)total * 2},
+                            {cells, d.cells, (size_t)total * 12}};
     CourierLease lease;
     Courier* courier = c->courier;
     if (!courier) courier = lease.c = take_courier(&e);
     if (courier) e = deliver(courier, c->stream, outs, 5);
     if (e != cudaSuccess) {
         cudaStreamSynchronize(c->stream);
-        cleanup();
         return cuda_fail(e, "point download");
     }
-    cleanup();
-    L3D_CUDA(cudaStreamSynchronize(c->stream), "point download");
     return L3D_OK;
 }
 
@@ -2577,7 +2584,7 @@ int64_t l3d_cloud_launches(const l3d_cloud* c) { return c ? c->launches : -1; }
 void l3d_cloud_destroy(l3d_cloud* c) {
     if (!c) return;
     free_table(c->t, c->stream);
-    for (void* q : {(void*)c->counters, (void*)c->err, (void*)c->thumb, (void*)c->map, (void*)c->pts})
+    for (void* q : {(void*)c->state, (void*)c->thumb, (void*)c->map, (void*)c->pts})
         if (q) cudaFreeAsync(q, c->stream);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->done) cudaEventDestroy(c->done);
@@ -2598,24 +2605,6 @@ struct l3d_mesh {
 };
 
 namespace {
-
-/* Scratch buffers allocated and freed in the order of stream `s` (no device-wide wait), freed
- * when the holder goes out of scope. */
-struct DevBufs {
-    cudaStream_t s;
-    std::vector<void*> ptrs;
-    explicit DevBufs(cudaStream_t stream) : s(stream) {}
-    ~DevBufs() {
-        for (void* p : ptrs) cudaFreeAsync(p, s);
-    }
-    template <typename T>
-    cudaError_t get(T** p, size_t count) {
-        *p = nullptr;
-        cudaError_t e = pool_alloc((void**)p, std::max<size_t>(count, 1) * sizeof(T), s);
-        if (e == cudaSuccess) ptrs.push_back(*p);
-        return e;
-    }
-};
 
 /* `n` words of the device, after the work queued on `s`. */
 template <typename T>

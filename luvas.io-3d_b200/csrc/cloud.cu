@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "l3d_fmath.h"
 #include "l3d_internal.h"
 
@@ -45,14 +47,8 @@ __device__ __forceinline__ bool pack_key(double fx, double fy, double fz, unsign
 }
 
 /* Slot of the cell (claimed when new), or -1 after setting an error flag. */
-__device__ int claim(const L3dCloudTable& t, double cx, double cy, double cz, unsigned* used,
-                     int* err) {
-    unsigned long long key;
-    int ix, iy, iz;
-    if (!pack_key(floor(cx), floor(cy), floor(cz), &key, &ix, &iy, &iz)) {
-        atomicOr(err, L3D_CLOUD_ERR_RANGE);
-        return -1;
-    }
+__device__ int claim_key(const L3dCloudTable& t, unsigned long long key, int ix, int iy, int iz, unsigned* used,
+                         int* err) {
     const unsigned mask = (unsigned)t.capacity - 1u;
     unsigned slot = cell_hash(ix, iy, iz) & mask;
     for (int probe = 0; probe < t.capacity; probe++) {
@@ -71,6 +67,15 @@ __device__ int claim(const L3dCloudTable& t, double cx, double cy, double cz, un
     atomicOr(err, L3D_CLOUD_ERR_FULL);
     return -1;
 }
+__device__ int claim(const L3dCloudTable& t, double cx, double cy, double cz, unsigned* used, int* err) {
+    unsigned long long key;
+    int ix, iy, iz;
+    if (!pack_key(floor(cx), floor(cy), floor(cz), &key, &ix, &iy, &iz)) {
+        atomicOr(err, L3D_CLOUD_ERR_RANGE);
+        return -1;
+    }
+    return claim_key(t, key, ix, iy, iz, used, err);
+}
 
 __device__ __forceinline__ void accumulate(const L3dCloudTable& t, int slot, const double* v,
                                            unsigned n) {
@@ -80,48 +85,63 @@ __device__ __forceinline__ void accumulate(const L3dCloudTable& t, int slot, con
     atomicAdd(t.counts + slot, n);
 }
 
-__device__ void sample_of(const L3dCloudView& v, uint32_t value, double d, int x, int y, int W,
-                          int H, const uint8_t* __restrict__ rgb, double* p);
+__device__ void sample_of(const L3dCloudView& v, const double* code, uint32_t value, double d, int x, int y,
+                          const uint8_t* __restrict__ rgb, double* p);
 
 /* addDepthMap (depth-fusion.ts:42-74) for one pixel; unpackDepthSample (depth-maps.ts:66-85).
- * Neighbouring pixels mostly land in the same cell: the lanes of a warp that share a cell add
- * their samples up first (in lane order), and one of them claims the cell and adds the sum, so
- * the table sees one set of atomics per cell and warp instead of one per pixel. */
-__global__ void k_cloud_add_map(const L3dCloudTable t, double cell, const uint32_t* __restrict__ packed,
-                                int W, int H, const L3dCloudView v, const uint8_t* __restrict__ rgb,
-                                unsigned* used, int* err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t value = i < W * H ? __ldg(packed + i) : 0u;
+ * Neighbouring pixels mostly land in the same cell: a warp takes 8 x 4 pixels, and the lanes that share
+ * a cell add their samples up first (in lane order), so that one of them claims the cell and adds the
+ * sum: the table sees one set of atomics per cell and warp instead of one per pixel.  The samples meet in
+ * shared memory, where every group's first lane sums its own at the same time; passing them along by
+ * shuffles ran the groups of a warp (about fifteen) one after the other.  Bound by the table's atomics
+ * and FP64 issue: a map of 640x480 takes 19 us, 34 us with shuffles and a row of 32 pixels per warp. */
+constexpr int kMapX = 32, kMapY = 8;  /* pixels per block of 256 threads */
+
+__global__ void __launch_bounds__(256) k_cloud_add_map(const L3dCloudTable t, double cell,
+                                                       const uint32_t* __restrict__ packed, int W, int H,
+                                                       const L3dCloudView v, const uint8_t* __restrict__ rgb,
+                                                       unsigned* used, int* err) {
+    __shared__ double code[64];           /* the decoded values of a 6-bit normal component */
+    __shared__ double samples[256][9];
+    if (threadIdx.x < 64) code[threadIdx.x] = ((double)threadIdx.x / 63.0) * 2.0 - 1.0;
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int across = (W + kMapX - 1) / kMapX, by = blockIdx.x / across, bx = blockIdx.x - by * across;
+    const int x = bx * kMapX + (warp & 3) * 8 + (lane & 7);
+    const int y = by * kMapY + (warp >> 2) * 4 + (lane >> 3);
+    const uint32_t value = x < W && y < H ? __ldg(packed + (size_t)y * W + x) : 0u;
     const double d = value ? (double)l3d_f16_to_f32(value & 0xffffu) : 0.0;
-    double p[9];
     unsigned long long key = 0;
+    int ix = 0, iy = 0, iz = 0;
     bool valid = d > 0.0;
     if (valid) {
-        sample_of(v, value, d, i % W, i / W, W, H, rgb, p);
-        int ix, iy, iz;
+        double p[9];
+        sample_of(v, code, value, d, x, y, rgb, p);
         valid = pack_key(floor(p[0] / cell), floor(p[1] / cell), floor(p[2] / cell), &key, &ix, &iy, &iz);
         if (!valid) atomicOr(err, L3D_CLOUD_ERR_RANGE);
+#pragma unroll
+        for (int k = 0; k < 9; k++) samples[threadIdx.x][k] = p[k];
     }
     const unsigned active = __ballot_sync(0xffffffffu, valid);
     if (!valid) return;
     const unsigned group = __match_any_sync(active, key);
-    double s[9];
+    __syncwarp(active);
+    if (lane != __ffs(group) - 1) return;
+    double s[9] = {};
+    for (unsigned m = group; m; m &= m - 1u) {
+        const double* q = samples[(threadIdx.x & ~31u) + __ffs(m) - 1];
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-        double acc = 0.0;
-        for (unsigned m = group; m; m &= m - 1u) acc += __shfl_sync(group, p[k], __ffs(m) - 1);
-        s[k] = acc;
+        for (int k = 0; k < 9; k++) s[k] += q[k];
     }
-    if ((int)(threadIdx.x & 31u) != __ffs(group) - 1) return;
-    const int slot = claim(t, p[0] / cell, p[1] / cell, p[2] / cell, used, err);
+    const int slot = claim_key(t, key, ix, iy, iz, used, err);
     if (slot >= 0) accumulate(t, slot, s, (unsigned)__popc(group));
 }
 
 /* The world sample of one valid pixel (depth d > 0): position, normal, thumbnail colour. */
-__device__ void sample_of(const L3dCloudView& v, uint32_t value, double d, int x, int y, int W,
-                          int H, const uint8_t* __restrict__ rgb, double* p) {
-    const double ex = ((double)((value >> 16) & 63u) / 63.0) * 2.0 - 1.0;
-    const double ey = ((double)((value >> 22) & 63u) / 63.0) * 2.0 - 1.0;
+__device__ void sample_of(const L3dCloudView& v, const double* code, uint32_t value, double d, int x, int y,
+                          const uint8_t* __restrict__ rgb, double* p) {
+    const double ex = code[(value >> 16) & 63u];
+    const double ey = code[(value >> 22) & 63u];
     double nx = ex, ny = ey;
     const double nz = 1.0 - fabs(ex) - fabs(ey);
     if (nz < 0.0) {
@@ -144,9 +164,8 @@ __device__ void sample_of(const L3dCloudView& v, uint32_t value, double d, int x
     p[3] = R[0] * nx + R[3] * ny + R[6] * nzn;
     p[4] = R[1] * nx + R[4] * ny + R[7] * nzn;
     p[5] = R[2] * nx + R[5] * ny + R[8] * nzn;
-    const double sx = (double)v.tw / W, sy = (double)v.th / H;
-    const int tx = min(v.tw - 1, (int)floor((x + 0.5) * sx));
-    const int ty = min(v.th - 1, (int)floor((y + 0.5) * sy));
+    const int tx = min(v.tw - 1, (int)floor((x + 0.5) * v.sx));
+    const int ty = min(v.th - 1, (int)floor((y + 0.5) * v.sy));
     const uint8_t* c = rgb + ((size_t)ty * v.tw + tx) * 3;
     p[6] = c[0];
     p[7] = c[1];
@@ -181,15 +200,116 @@ __global__ void k_cloud_rebin(const L3dCloudTable from, const L3dCloudTable to, 
     if (slot >= 0) accumulate(to, slot, p, n);
 }
 
-/* cloud(minSupport) (point-accumulator.ts:114-143), in three steps on the device: the cell keys
- * and slots of the slots with enough support (arbitrary order), the pairs sorted by key, then
- * the averaged points gathered in key order (cells ascending: z, then y, then x). */
+/* cloud(minSupport) (point-accumulator.ts:114-143): the averaged points of the slots with enough support,
+ * cells ascending (z, then y, then x).  The cells are distinct, so where their box is not much larger
+ * than their number a point's place is the number of cells before it in the box: a bit per cell of the
+ * box, a prefix sum over groups of 256 bits, and every slot writes its point where it belongs.  100
+ * thousand points in a box of 18 million cells take 55 us; sorting their (key, slot) pairs, which wide
+ * boxes still do, took 208 us. */
+__device__ __forceinline__ bool counted(const L3dCloudTable& t, int s, unsigned min_support, unsigned long long* key) {
+    if (s >= t.capacity) return false;
+    *key = t.keys[s];
+    return *key != kEmpty && t.counts[s] >= min_support;
+}
+
+/* The number of counted slots and the box of their (biased) cells. */
+__global__ void __launch_bounds__(256) k_cloud_box(const L3dCloudTable t, unsigned min_support, L3dCloudState* state) {
+    __shared__ unsigned part[7];
+    if (threadIdx.x < 7) part[threadIdx.x] = threadIdx.x < 3 ? ~0u : 0u;
+    __syncthreads();
+    unsigned n = 0, lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0u, 0u, 0u};
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < t.capacity; s += gridDim.x * blockDim.x) {
+        unsigned long long key;
+        if (!counted(t, s, min_support, &key)) continue;
+        n++;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const unsigned c = (unsigned)(key >> (21 * k)) & 0x1fffffu;
+            lo[k] = min(lo[k], c);
+            hi[k] = max(hi[k], c);
+        }
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        lo[k] = __reduce_min_sync(0xffffffffu, lo[k]);
+        hi[k] = __reduce_max_sync(0xffffffffu, hi[k]);
+    }
+    if ((threadIdx.x & 31) == 0 && n) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            atomicMin(&part[k], lo[k]);
+            atomicMax(&part[3 + k], hi[k]);
+        }
+        atomicAdd(&part[6], n);
+    }
+    __syncthreads();
+    if (!part[6]) return;
+    if (threadIdx.x < 3) atomicMin(&state->lo[threadIdx.x], part[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&state->hi[threadIdx.x - 3], part[threadIdx.x]);
+    else if (threadIdx.x == 6) atomicAdd(&state->total, part[6]);
+}
+
+__device__ __forceinline__ unsigned long long place_of(const L3dCloudBox& b, unsigned long long key) {
+    const unsigned x = (unsigned)key & 0x1fffffu, y = (unsigned)(key >> 21) & 0x1fffffu, z = (unsigned)(key >> 42) & 0x1fffffu;
+    return ((unsigned long long)(z - b.lo[2]) * b.dims[1] + (y - b.lo[1])) * b.dims[0] + (x - b.lo[0]);
+}
+
+__global__ void k_cloud_bits(const L3dCloudTable t, unsigned min_support, const L3dCloudBox b, uint32_t* bits) {
+    unsigned long long key;
+    if (!counted(t, blockIdx.x * blockDim.x + threadIdx.x, min_support, &key)) return;
+    const unsigned long long i = place_of(b, key);
+    atomicOr(bits + (i >> 5), 1u << (i & 31));
+}
+
+/* Set bits per group of 256. */
+__global__ void k_cloud_groups(const uint32_t* bits, long long groups, uint32_t* count) {
+    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= groups) return;
+    const uint4 a = ((const uint4*)bits)[g * 2], b = ((const uint4*)bits)[g * 2 + 1];
+    count[g] = __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w) + __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
+}
+
+/* Point o: the means of slot s. */
+__device__ __forceinline__ void put_point(const L3dCloudTable& t, uint32_t s, unsigned long long key, size_t o,
+                                          const L3dCloudOut& out) {
+    const unsigned n = t.counts[s];
+    const double* sm = t.sums + (size_t)s * 9;
+    const double dn = (double)n;
+    for (int j = 0; j < 3; j++) out.pos[o * 3 + j] = (float)(sm[j] / dn);
+    double len = sqrt(sm[3] * sm[3] + sm[4] * sm[4] + sm[5] * sm[5]);
+    if (!(len != 0.0)) len = 1.0;
+    for (int j = 0; j < 3; j++) out.nrm[o * 3 + j] = (float)(sm[3 + j] / len);
+    for (int j = 0; j < 3; j++) {
+        /* Uint8Array store: truncation, then modulo 256 */
+        double c = trunc(sm[6 + j] / dn);
+        c = c - 256.0 * floor(c / 256.0);
+        out.col[o * 3 + j] = (uint8_t)c;
+    }
+    out.support[o] = (uint16_t)min(n, 65535u);
+    for (int j = 0; j < 3; j++)
+        out.cells[o * 3 + j] = (int32_t)((long long)((key >> (21 * j)) & 0x1FFFFFull) - kBias);
+}
+
+__global__ void k_cloud_emit_placed(const L3dCloudTable t, unsigned min_support, const L3dCloudBox b,
+                                    const uint32_t* bits, const uint32_t* before, const L3dCloudOut out) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long key;
+    if (!counted(t, s, min_support, &key)) return;
+    const unsigned long long i = place_of(b, key);
+    const unsigned long long g = i >> 8;
+    uint32_t o = before[g];
+    for (unsigned long long w = g * 8; w < i >> 5; w++) o += __popc(bits[w]);
+    o += __popc(bits[i >> 5] & ((1u << (i & 31)) - 1u));
+    put_point(t, (uint32_t)s, key, o, out);
+}
+
+/* The cell keys and slots of the counted slots, in any order (for the sort). */
 __global__ void k_cloud_emit_keys(const L3dCloudTable t, unsigned min_support, unsigned* count,
                                   unsigned long long* keys, uint32_t* slots) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= t.capacity) return;
-    const unsigned long long key = t.keys[s];
-    if (key == kEmpty || t.counts[s] < min_support) return;
+    unsigned long long key;
+    if (!counted(t, s, min_support, &key)) return;
     const unsigned o = atomicAdd(count, 1u);
     keys[o] = key;
     slots[o] = (uint32_t)s;
@@ -197,28 +317,9 @@ __global__ void k_cloud_emit_keys(const L3dCloudTable t, unsigned min_support, u
 
 __global__ void k_cloud_emit_sorted(const L3dCloudTable t, unsigned total,
                                     const unsigned long long* __restrict__ keys,
-                                    const uint32_t* __restrict__ slots, float* pos, float* nrm,
-                                    uint8_t* col, uint16_t* support, int32_t* cells) {
+                                    const uint32_t* __restrict__ slots, const L3dCloudOut out) {
     const unsigned o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= total) return;
-    const uint32_t s = slots[o];
-    const unsigned long long key = keys[o];
-    const unsigned n = t.counts[s];
-    const double* sm = t.sums + (size_t)s * 9;
-    const double dn = (double)n;
-    for (int j = 0; j < 3; j++) pos[(size_t)o * 3 + j] = (float)(sm[j] / dn);
-    double len = sqrt(sm[3] * sm[3] + sm[4] * sm[4] + sm[5] * sm[5]);
-    if (!(len != 0.0)) len = 1.0;
-    for (int j = 0; j < 3; j++) nrm[(size_t)o * 3 + j] = (float)(sm[3 + j] / len);
-    for (int j = 0; j < 3; j++) {
-        /* Uint8Array store: truncation, then modulo 256 */
-        double c = trunc(sm[6 + j] / dn);
-        c = c - 256.0 * floor(c / 256.0);
-        col[(size_t)o * 3 + j] = (uint8_t)c;
-    }
-    support[o] = (uint16_t)min(n, 65535u);
-    for (int j = 0; j < 3; j++)
-        cells[(size_t)o * 3 + j] = (int32_t)((long long)((key >> (21 * j)) & 0x1FFFFFull) - kBias);
+    if (o < total) put_point(t, slots[o], keys[o], o, out);
 }
 
 /* Bitonic sort of n = 2^m (key, value) pairs, m >= 11, ascending by key.  Stages with a
@@ -277,14 +378,13 @@ __global__ void k_bitonic_global(unsigned long long* keys, uint32_t* vals, unsig
     order_pair(keys, vals, i, i + j, (i & k) == 0);
 }
 
-__global__ void k_cloud_clear(L3dCloudTable t) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= t.capacity) return;
-    t.keys[s] = kEmpty;
-    t.counts[s] = 0u;
-    double* sm = t.sums + (size_t)s * 9;
-#pragma unroll
-    for (int j = 0; j < 9; j++) sm[j] = 0.0;
+/* Empty keys, zero sums and counts, 16 bytes per store (capacity is a power of two, at least 2^16). */
+__global__ void __launch_bounds__(256) k_cloud_clear(L3dCloudTable t) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = (long long)gridDim.x * blockDim.x;
+    const long long keys = t.capacity / 2, sums = (long long)t.capacity * 9 / 2, counts = t.capacity / 4;
+    for (long long k = i; k < keys; k += n) ((ulonglong2*)t.keys)[k] = make_ulonglong2(kEmpty, kEmpty);
+    for (long long k = i; k < sums; k += n) ((double2*)t.sums)[k] = make_double2(0.0, 0.0);
+    for (long long k = i; k < counts; k += n) ((uint4*)t.counts)[k] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 inline unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
@@ -292,7 +392,7 @@ inline unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
 }  // namespace
 
 cudaError_t l3d_launch_cloud_clear(const L3dCloudTable& t, cudaStream_t stream) {
-    k_cloud_clear<<<blocks_for(t.capacity), 256, 0, stream>>>(t);
+    k_cloud_clear<<<(unsigned)std::min((long long)blocks_for(t.capacity), 148ll * 8), 256, 0, stream>>>(t);
     return cudaGetLastError();
 }
 
@@ -300,8 +400,8 @@ cudaError_t l3d_launch_cloud_add_map(const L3dCloudTable& t, double cell, const 
                                      int W, int H, const L3dCloudView& v, const uint8_t* rgb,
                                      unsigned* used, int* err, cudaStream_t stream) {
     if ((long long)W * H == 0) return cudaSuccess;
-    k_cloud_add_map<<<blocks_for((long long)W * H), 256, 0, stream>>>(t, cell, packed, W, H, v, rgb,
-                                                                      used, err);
+    const long long blocks = (long long)((W + kMapX - 1) / kMapX) * ((H + kMapY - 1) / kMapY);
+    k_cloud_add_map<<<(unsigned)blocks, 256, 0, stream>>>(t, cell, packed, W, H, v, rgb, used, err);
     return cudaGetLastError();
 }
 
@@ -352,12 +452,37 @@ cudaError_t l3d_launch_cloud_sort(unsigned long long* keys, uint32_t* slots, uns
     return cudaGetLastError();
 }
 
+cudaError_t l3d_launch_cloud_box(const L3dCloudTable& t, unsigned min_support, L3dCloudState* state,
+                                 cudaStream_t stream) {
+    const unsigned blocks = (unsigned)std::min((long long)blocks_for(t.capacity), 148ll * 8);
+    k_cloud_box<<<blocks, 256, 0, stream>>>(t, min_support, state);
+    return cudaGetLastError();
+}
+
+long long l3d_cloud_box_groups(const L3dCloudBox& b, unsigned total) {
+    /* the box's bits are cleared and read once: up to 4096 of them a point cost less than the sort, and
+     * 128 MB are scratch enough */
+    const double cells = (double)b.dims[0] * b.dims[1] * b.dims[2];
+    if (cells > 4096.0 * total || cells > (double)(1ll << 30)) return 0;
+    return ((long long)cells + 255) / 256;
+}
+
+cudaError_t l3d_launch_cloud_emit_placed(const L3dCloudTable& t, unsigned min_support, const L3dCloudBox& b,
+                                         long long groups, uint32_t* bits, uint32_t* before, uint32_t* scratch,
+                                         const L3dCloudOut& out, cudaStream_t stream) {
+    cudaError_t e = cudaMemsetAsync(bits, 0, (size_t)groups * 32, stream);
+    if (e != cudaSuccess) return e;
+    k_cloud_bits<<<blocks_for(t.capacity), 256, 0, stream>>>(t, min_support, b, bits);
+    k_cloud_groups<<<blocks_for(groups), 256, 0, stream>>>(bits, groups, before);
+    if ((e = l3d_scan_exclusive(before, before, groups, scratch, nullptr, stream)) != cudaSuccess) return e;
+    k_cloud_emit_placed<<<blocks_for(t.capacity), 256, 0, stream>>>(t, min_support, b, bits, before, out);
+    return cudaGetLastError();
+}
+
 cudaError_t l3d_launch_cloud_emit_sorted(const L3dCloudTable& t, unsigned total,
                                          const unsigned long long* keys, const uint32_t* slots,
-                                         float* pos, float* nrm, uint8_t* col, uint16_t* support,
-                                         int32_t* cells, cudaStream_t stream) {
+                                         const L3dCloudOut& out, cudaStream_t stream) {
     if (total == 0) return cudaSuccess;
-    k_cloud_emit_sorted<<<blocks_for(total), 256, 0, stream>>>(t, total, keys, slots, pos, nrm, col,
-                                                              support, cells);
+    k_cloud_emit_sorted<<<blocks_for(total), 256, 0, stream>>>(t, total, keys, slots, out);
     return cudaGetLastError();
 }

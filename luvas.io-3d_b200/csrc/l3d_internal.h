@@ -324,6 +324,23 @@ struct L3dCloudView {
     double R[9];
     double t[3];
     int tw, th;
+    double sx, sy;             /* thumbnail pixels per map pixel: tw / W, th / H */
+};
+/* A cloud's words on the device. */
+struct L3dCloudState {
+    unsigned used;             /* claimed slots */
+    int err;
+    unsigned total, hi[3];     /* read-back: counted slots and the box of their biased cells (zeroed, */
+    unsigned lo[3];            /* all ones) */
+};
+struct L3dCloudBox {
+    unsigned lo[3], dims[3];
+};
+struct L3dCloudOut {
+    float *pos, *nrm;
+    uint8_t* col;
+    uint16_t* support;
+    int32_t* cells;
 };
 
 enum { L3D_CLOUD_ERR_RANGE = 1, L3D_CLOUD_ERR_FULL = 2 };
@@ -336,9 +353,17 @@ cudaError_t l3d_launch_cloud_add_points(const L3dCloudTable& t, double cell, con
                                         long long n, unsigned* used, int* err, cudaStream_t stream);
 cudaError_t l3d_launch_cloud_rebin(const L3dCloudTable& from, const L3dCloudTable& to, double cell,
                                    unsigned* used, int* err, cudaStream_t stream);
-/* cloud read-back: (key, slot) of the slots with at least min_support samples, appended at
- * *count; the pairs sorted by key on the device (n = l3d_cloud_sort_length(total) entries,
- * padded); the points gathered in key order. */
+/* cloud read-back: state->total, hi, lo of the slots with at least min_support samples; then either the
+ * points placed by their cell's number in the box (groups = l3d_cloud_box_groups > 0: 8 words of bits
+ * and one of `before` per group, scratch of l3d_scan_scratch(groups); three launches and a scan), or
+ * (key, slot) pairs appended at *count, sorted by key (n = l3d_cloud_sort_length(total) entries,
+ * padded) and the points gathered in key order. */
+cudaError_t l3d_launch_cloud_box(const L3dCloudTable& t, unsigned min_support, L3dCloudState* state,
+                                 cudaStream_t stream);
+long long l3d_cloud_box_groups(const L3dCloudBox& b, unsigned total);
+cudaError_t l3d_launch_cloud_emit_placed(const L3dCloudTable& t, unsigned min_support, const L3dCloudBox& b,
+                                         long long groups, uint32_t* bits, uint32_t* before, uint32_t* scratch,
+                                         const L3dCloudOut& out, cudaStream_t stream);
 cudaError_t l3d_launch_cloud_emit_keys(const L3dCloudTable& t, unsigned min_support,
                                        unsigned* count, unsigned long long* keys, uint32_t* slots,
                                        cudaStream_t stream);
@@ -347,8 +372,7 @@ cudaError_t l3d_launch_cloud_sort(unsigned long long* keys, uint32_t* slots, uns
                                   unsigned n, long long* launches, cudaStream_t stream);
 cudaError_t l3d_launch_cloud_emit_sorted(const L3dCloudTable& t, unsigned total,
                                          const unsigned long long* keys, const uint32_t* slots,
-                                         float* pos, float* nrm, uint8_t* col, uint16_t* support,
-                                         int32_t* cells, cudaStream_t stream);
+                                         const L3dCloudOut& out, cudaStream_t stream);
 
 /* ---- prefix sums (scan.cu) ---- */
 
