@@ -307,6 +307,7 @@ bool l3d_tsdf_grid_of(const l3d_tsdf_desc* d, bool pool_coords_given, L3dTsdfGri
     }
     g.voxel = (float)d->voxel;
     g.mu = (float)d->truncation;
+    g.inv_mu = 1.0f / g.mu;
     g.prior_weight = (float)d->prior_weight;
     g.max_weight = (float)d->max_weight;
     g.max_q = (unsigned)rintf(g.max_weight * 256.0f);
@@ -1647,7 +1648,7 @@ struct l3d_tsdf {
     int32_t* list = nullptr;          /* 1 + bricks: kept bricks of a one-view integration */
     uint32_t* sweep = nullptr;        /* the sweep's brick list: flags, prefix (bricks + 1 each),
                                          list (bricks), scan scratch */
-    uint8_t* super = nullptr;         /* super-brick flags of the visibility pass, super_cap */
+    uint32_t* super = nullptr;        /* (super-brick, view) list of the visibility pass, super_cap words */
     long long super_cap = 0;
     cudaEvent_t read_done = nullptr;  /* after the copies of an asynchronous read-back */
     bool read_pending = false;
@@ -1728,13 +1729,13 @@ int after_read(l3d_tsdf* t) {
 }
 
 int ensure_super(l3d_tsdf* t, int n_views) {
-    const long long n = l3d_tsdf_super_flags(t->g, n_views);
+    const long long n = l3d_tsdf_super_pairs(t->g, n_views) + 1;
     if (t->super_cap >= n) return L3D_OK;
-    L3D_CUDA(cudaStreamSynchronize(t->stream), "super-brick flags: wait");
-    L3D_CUDA(cudaFree(t->super), "super-brick flags: free");
+    L3D_CUDA(cudaStreamSynchronize(t->stream), "super-brick list: wait");
+    L3D_CUDA(cudaFree(t->super), "super-brick list: free");
     t->super = nullptr;
     t->super_cap = 0;
-    L3D_CUDA(cudaMalloc(&t->super, (size_t)n), "super-brick flags");
+    L3D_CUDA(dalloc(&t->super, (size_t)n), "super-brick list");
     t->super_cap = n;
     return L3D_OK;
 }
@@ -1987,6 +1988,7 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
     L3D_CUDA(cudaMemcpyAsync(t->views, t->views_host, (size_t)n * sizeof(L3dTsdfView), cudaMemcpyHostToDevice, t->stream), "view upload");
     L3D_CUDA(cudaMemcpyAsync(t->depth_ptrs, t->ptrs_host, (size_t)n * sizeof(void*), cudaMemcpyHostToDevice, t->stream), "view upload");
     L3D_CUDA(cudaEventRecord(t->staged, t->stream), "event record");
+    const bool ordinary = l3d_tsdf_ordinary(t->g, t->views_host, n);
     cudaError_t e;
     if (counts_out) {
         /* visibleBricks alone: visible voxel-views and updates; then the depth-aware mask: the
@@ -2008,7 +2010,7 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
                                       t->normals, counts + 2, t->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(host, counts, sizeof(host), cudaMemcpyDeviceToHost, t->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
-        t->launches += 5 + (l3d_tsdf_super_flags(t->g, n) > 0 ? 1 : 0);
+        t->launches += 4 + l3d_tsdf_visible_launches(t->g, n);
         cudaFreeAsync(counts, t->stream);
         if (e != cudaSuccess) return cuda_fail(e, "update count");
         if (host[3] != host[1])
@@ -2027,12 +2029,12 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
     if (e == cudaSuccess)
         e = l3d_launch_tsdf_brick_list(t->g, n, t->mask, sweep_flags(t), sweep_prefix(t), sweep_list(t),
                                        sweep_scratch(t), t->stream);
-    t->launches += 4 + (l3d_tsdf_super_flags(t->g, n) > 0 ? 1 : 0) + l3d_scan_launches(t->g.bricks + 1);
+    t->launches += 3 + l3d_tsdf_visible_launches(t->g, n) + l3d_scan_launches(t->g.bricks + 1);
     if (e != cudaSuccess) return cuda_fail(e, "visibility launch");
     if (!tsdf_out && !weight_out) {
         e = l3d_launch_tsdf_many_list(t->g, t->views, n, t->coords, t->mask, t->depth_ptrs, t->priors,
                                       t->normals, t->tsdf, t->weight, t->q8, sweep_prefix(t),
-                                      sweep_list(t), 0, l3d_tsdf_sweep_units(t->g, nullptr, nullptr),
+                                      sweep_list(t), ordinary, 0, l3d_tsdf_sweep_units(t->g, nullptr, nullptr),
                                       t->stream);
         t->launches++;
         if (e != cudaSuccess) return cuda_fail(e, "integrate launch");
@@ -2054,7 +2056,7 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
             const long long q1 = std::min(layers, i * per + per) * lu;
             e = l3d_launch_tsdf_many_list(t->g, t->views, n, t->coords, t->mask, t->depth_ptrs,
                                           t->priors, t->normals, t->tsdf, t->weight, t->q8,
-                                          sweep_prefix(t), sweep_list(t), q0, q1, t->stream);
+                                          sweep_prefix(t), sweep_list(t), ordinary, q0, q1, t->stream);
             t->launches += q1 > q0 ? 1 : 0;
             if (e != cudaSuccess) return cuda_fail(e, "integrate launch");
             L3D_CUDA(cudaEventRecord(t->slab_done[i], t->stream), "event record");

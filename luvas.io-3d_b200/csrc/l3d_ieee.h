@@ -39,4 +39,18 @@ __device__ __forceinline__ float l3d_div_normal(float a, float b) {
     return fmaf(fmaf(-b, q, a), y, q);
 }
 
+/* a / b, given y = 1.0f / b rounded, under the conditions of l3d_div_normal (a zero a excepted when its
+ * sign matters: -0 / b gives +0). */
+__device__ __forceinline__ float l3d_div_by(float a, float b, float y) {
+    const float q = a * y;
+    return fmaf(fmaf(-b, q, a), y, q);
+}
+
+/* rintf(x) as an index: for an integer n <= 2^22, the result is below n exactly when rintf(x) (ties to
+ * even) lies in [0, n), and is then rintf(x).  Adding 1.5 x 2^23 leaves the rounded integer in the sum's
+ * low bits; a sum outside [1.5 x 2^23, 1.5 x 2^23 + n), NaN included, has bits outside theirs. */
+__device__ __forceinline__ unsigned l3d_rint_index(float x) {
+    return __float_as_uint(x + 12582912.0f) - 0x4b400000u;
+}
+
 #endif

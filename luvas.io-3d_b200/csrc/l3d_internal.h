@@ -64,6 +64,7 @@ struct L3dTsdfGrid {
     float origin[3];
     float voxel;
     float mu;
+    float inv_mu;              /* 1 / mu in f32 */
     float prior_weight;
     float max_weight;
     unsigned max_q;            /* rint(max_weight * 256) for Q8.8 weights */
@@ -84,6 +85,11 @@ struct L3dTsdfGrid {
 bool l3d_tsdf_grid_of(const l3d_tsdf_desc* d, bool pool_coords_given, L3dTsdfGrid* out, char* why,
                       size_t why_size);
 L3dTsdfView l3d_tsdf_view_of(const l3d_integration_view& v);
+
+/* Whether the numbers of these views' integration stay ordinary (tsdf.cu): |camera coordinates| < 2^50,
+ * mu in [2^-60, 2^60], map sides at most 2^22.  The kernels over lists of kept bricks rely on it; what
+ * is not ordinary goes through the general ones. */
+bool l3d_tsdf_ordinary(const L3dTsdfGrid& g, const L3dTsdfView* views, int n);
 
 /* ---- launchers (stereo.cu / stereo_fast.cu / tsdf.cu); each returns cudaGetLastError() ---- */
 
@@ -202,17 +208,15 @@ long long l3d_depth_tile_count(int W, int H);
 cudaError_t l3d_launch_depth_tiles(const L3dTsdfView* views_dev, int n_views,
                                    const uint32_t* const* depth_ptrs_dev, const float* priors,
                                    float* tiles, long long max_tiles, cudaStream_t stream);
-/* brick mask of n views with the depth-aware cull: visibleBricks and, where `tiles` is given
- * (l3d_launch_depth_tiles first), not provably behind every depth of its footprint by more than
- * the truncation band (such a brick has no voxel that updates) */
+/* brick mask of n views with the depth-aware cull: visibleBricks and not provably behind every depth
+ * of its footprint (`tiles`: l3d_launch_depth_tiles first) by more than the truncation band (such a
+ * brick has no voxel that updates).  A dense grid tests blocks of 4^3 bricks per view first and lists
+ * those to look into in `pairs` (1 + l3d_tsdf_super_pairs words; 0 pairs: a brick pool, no list). */
 cudaError_t l3d_launch_tsdf_visible_depth(const L3dTsdfGrid& g, const L3dTsdfView* views_dev, int n_views,
-                                          const int32_t* coords, const float* tiles, uint8_t* super,
+                                          const int32_t* coords, const float* tiles, uint32_t* pairs,
                                           uint8_t* mask, cudaStream_t stream);
-/* Bytes of the super-brick flags l3d_launch_tsdf_visible_depth uses on a dense grid (0 for a
- * brick pool, which gets no super-brick pass; `super` may then be NULL).  With `super` and
- * `tiles` it first tests blocks of 4^3 bricks per view and skips the bricks of those behind the
- * depths (one launch more). */
-long long l3d_tsdf_super_flags(const L3dTsdfGrid& g, int n_views);
+int l3d_tsdf_visible_launches(const L3dTsdfGrid& g, int n_views);
+long long l3d_tsdf_super_pairs(const L3dTsdfGrid& g, int n_views);
 /* counts[0] += visible voxel-views, counts[1] += voxel-updates of a many-view integration */
 cudaError_t l3d_launch_tsdf_count(const L3dTsdfGrid& g, const L3dTsdfView* views_dev, int n_views,
                                   const int32_t* coords, const uint8_t* mask,
@@ -232,7 +236,7 @@ cudaError_t l3d_launch_tsdf_many_list(const L3dTsdfGrid& g, const L3dTsdfView* v
                                       int n_views, const int32_t* coords, const uint8_t* mask,
                                       const uint32_t* const* depth_ptrs_dev, const float* priors,
                                       const float4* normals, float* tsdf, void* weight, int q8,
-                                      const uint32_t* prefix, const int32_t* list,
+                                      const uint32_t* prefix, const int32_t* list, bool ordinary,
                                       long long q_begin, long long q_end, cudaStream_t stream);
 cudaError_t l3d_launch_tsdf_many(const L3dTsdfGrid& g, const L3dTsdfView* views_dev, int n_views,
                                  const int32_t* coords, const uint8_t* mask,

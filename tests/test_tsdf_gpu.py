@@ -294,3 +294,38 @@ def test_sweep_with_prior_and_depth_cull_bit_exact(scene, q8):
         t, w = g.read()
         assert_bit_equal(t.reshape(-1), o.tsdf, f"tsdf ({what})")
         assert_bit_equal(w.reshape(-1), o.weight, f"weight ({what})")
+
+
+@pytest.mark.parametrize("q8", [False, True])
+@pytest.mark.parametrize("dims,mu", [((36, 35, 33), 0.12), ((33, 41, 31), 0.12), ((36, 35, 33), 2.0**60),
+                                     ((36, 35, 33), 2.0**61)])
+def test_range_limits_and_remainders_bit_exact(scene, dims, mu, q8):
+    """Grids whose blocks of 4^3 bricks and whose fill (41943 voxels) end in remainders, truncations on
+    both sides of the line up to which the divisions are known to stay among normal numbers, and depths
+    beyond it (infinite samples and priors): per view and as a sweep, equal to the oracle."""
+    views, maps = scene
+    W, H = 120, 90
+    voxel, origin = 0.07, (-1.3, -1.2, -1.1)
+    maps = [m.copy() for m in maps]
+    maps[1][::7, ::5] = 0x7C00 | (maps[1][::7, ::5] & 0xFFFF0000)
+    prior = np.where(maps[2] == 0, 1.9, 0.0).astype(np.float32)
+    prior[::3] = np.inf
+    prior[1::3, ::2] = 3e38
+    o = oracle.Tsdf(W, H, voxel, origin, mu, dense=dims, weight_q8=q8)
+    a = TsdfVolume(W, H, voxel, origin, dense=dims, truncation=mu, weight_q8=q8)
+    b = TsdfVolume(W, H, voxel, origin, dense=dims, truncation=mu, weight_q8=q8)
+    gv = []
+    for i, (v, m) in enumerate(zip(views, maps)):
+        pr = prior if i == 2 else None
+        o.integrate(view_kw(v, prior=pr), m)
+        a.integrate(gpu_view(v, prior=pr), depth=m)
+        gv.append(gpu_view(v, prior=pr))
+    b.integrate_many(gv, depths=np.stack(maps))
+    for g, what in ((a, "per view"), (b, "sweep")):
+        t, w = g.read()
+        assert_bit_equal(t.reshape(-1), o.tsdf, f"tsdf ({what})")
+        assert_bit_equal(w.reshape(-1), o.weight, f"weight ({what})")
+        g.reset()
+        t, w = g.read()
+        assert np.all(t == 1.0) and np.all(w == 0)
+    assert (o.weight > 0).sum() > 1000
