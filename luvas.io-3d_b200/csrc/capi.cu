@@ -2034,7 +2034,7 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
     if (!tsdf_out && !weight_out) {
         e = l3d_launch_tsdf_many_list(t->g, t->views, n, t->coords, t->mask, t->depth_ptrs, t->priors,
                                       t->normals, t->tsdf, t->weight, t->q8, sweep_prefix(t),
-                                      sweep_list(t), ordinary, 0, l3d_tsdf_sweep_units(t->g, nullptr, nullptr),
+                                      sweep_list(t), sweep_scratch(t), ordinary, 0, l3d_tsdf_sweep_units(t->g, nullptr, nullptr),
                                       t->stream);
         t->launches++;
         if (e != cudaSuccess) return cuda_fail(e, "integrate launch");
@@ -2056,7 +2056,7 @@ static int integrate_many(l3d_tsdf* t, const l3d_stereo* src, const int32_t* lay
             const long long q1 = std::min(layers, i * per + per) * lu;
             e = l3d_launch_tsdf_many_list(t->g, t->views, n, t->coords, t->mask, t->depth_ptrs,
                                           t->priors, t->normals, t->tsdf, t->weight, t->q8,
-                                          sweep_prefix(t), sweep_list(t), ordinary, q0, q1, t->stream);
+                                          sweep_prefix(t), sweep_list(t), sweep_scratch(t), ordinary, q0, q1, t->stream);
             t->launches += q1 > q0 ? 1 : 0;
             if (e != cudaSuccess) return cuda_fail(e, "integrate launch");
             L3D_CUDA(cudaEventRecord(t->slab_done[i], t->stream), "event record");
@@ -2146,7 +2146,7 @@ static int tsdf_depth_run(l3d_tsdf* t, const l3d_integration_view* view, int32_t
     }
     /* the caller's buffers may be the handle's own volume: after its pending read-back */
     if (t->read_pending) L3D_CUDA(cudaStreamWaitEvent(st, t->read_done, 0), "stream wait");
-    cudaError_t e = l3d_launch_tsdf_depth(t->g, v, t->coords, t->mask, packed, depth, prior, tsdf_in,
+    cudaError_t e = l3d_launch_tsdf_depth(t->g, v, t->coords, t->mask, packed, depth, prior, t->normals, tsdf_in,
                                           weight_in, tsdf_out, weight_out, grad_tsdf_out,
                                           grad_weight_out, grad_depth, grad_tsdf_in, grad_weight_in,
                                           t->q8, st);

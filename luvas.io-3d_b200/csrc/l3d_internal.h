@@ -236,7 +236,8 @@ cudaError_t l3d_launch_tsdf_many_list(const L3dTsdfGrid& g, const L3dTsdfView* v
                                       int n_views, const int32_t* coords, const uint8_t* mask,
                                       const uint32_t* const* depth_ptrs_dev, const float* priors,
                                       const float4* normals, float* tsdf, void* weight, int q8,
-                                      const uint32_t* prefix, const int32_t* list, bool ordinary,
+                                      const uint32_t* prefix, const int32_t* list, uint32_t* next,
+                                      bool ordinary,
                                       long long q_begin, long long q_end, cudaStream_t stream);
 cudaError_t l3d_launch_tsdf_many(const L3dTsdfGrid& g, const L3dTsdfView* views_dev, int n_views,
                                  const int32_t* coords, const uint8_t* mask,
@@ -307,7 +308,7 @@ cudaError_t l3d_launch_ncc_grad(const L3dGradDev& d, const L3dGradView* views_de
  * adjoint.  Two launches. */
 cudaError_t l3d_launch_tsdf_depth(const L3dTsdfGrid& g, const L3dTsdfView& v, const int32_t* coords,
                                   uint8_t* mask, const uint32_t* depth, const float* depthf,
-                                  const float* prior, const float* tsdf_in, const void* weight_in,
+                                  const float* prior, const float4* normals, const float* tsdf_in, const void* weight_in,
                                   float* tsdf_out, void* weight_out, const float* grad_tsdf_out,
                                   const float* grad_weight_out, float* grad_depth,
                                   float* grad_tsdf_in, float* grad_weight_in, int q8,

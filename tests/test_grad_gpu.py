@@ -15,8 +15,8 @@ from helpers import arc_workload
 
 torch = pytest.importorskip("torch")
 
-from luvas3d import (DTYPE_F16, FORM_FAST, DenseStereo, IntegrationView, StereoOptions,  # noqa: E402
-                     TsdfVolume)
+from luvas3d import (DTYPE_F16, FORM_FAST, BrickGrid, DenseStereo, IntegrationView,  # noqa: E402
+                     StereoOptions, TsdfVolume)
 from luvas3d import grad as G  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -205,6 +205,45 @@ def test_tsdf_forward_depth_equals_integrate(tsdf_case, q8):
     got_w = w1.cpu().numpy()
     assert np.array_equal(got_w.view(np.uint16) if q8 else got_w.view(np.uint32),
                           want_w.reshape(-1).view(np.uint16 if q8 else np.uint32))
+
+
+@pytest.mark.parametrize("q8", [False, True])
+@pytest.mark.parametrize("dims", [(48, 40, 48), (44, 21, 29), (37, 21, 30), None])
+@pytest.mark.parametrize("mu,offset", [(0.15, 0), (0.15, 1), (2.0**61, 0)])
+def test_tsdf_depth_forms_agree(tsdf_case, q8, dims, mu, offset):
+    """Four voxels per access, one, and the general divisions (a truncation beyond the range of the others;
+    grids and pools; tensors off the 16-byte boundary): two chained updates equal the handle's own, and
+    the state's gradient equals the closed form wT = W0 / W1 there."""
+    views, packed, unpacked = tsdf_case[:3]
+    grid = BrickGrid((-1.2, -1.0, -1.2), 0.05, (2.4, 2.0, 2.4))
+    grid.marks[1::3] = 1
+    vol = TsdfVolume(96, 72, 0.05, (-1.2, -1.0, -1.2), dense=dims, layout=None if dims else grid.build(),
+                     truncation=mu, weight_q8=q8)
+    n = vol.voxels
+    wt = torch.int16 if q8 else torch.float32
+    t = torch.ones(n + offset, device="cuda")[offset:].requires_grad_(True)
+    w = torch.zeros(n + offset, dtype=wt, device="cuda")[offset:]
+    pk, dep = _cuda(packed.view(np.int32)), _cuda(unpacked)
+    first = None
+    for v in (views[0], views[1]):
+        iv = IntegrationView(v.intrinsics, v.pose, 5.0, None, 1.5)
+        vol.integrate(iv, depth=packed)
+        want_t, want_w = vol.read()
+        if first is not None:
+            t, w = (torch.cat([torch.zeros(offset, dtype=a.dtype, device="cuda"), a.detach()])[offset:] for a in first)
+            t.requires_grad_(True)
+        first = t1, w1 = G.integrate_depth(vol, iv, pk, dep, t, w)
+        assert np.array_equal(t1.detach().cpu().numpy().view(np.uint32), want_t.reshape(-1).view(np.uint32))
+        assert np.array_equal(w1.detach().cpu().numpy().view(np.uint16 if q8 else np.uint32),
+                              want_w.reshape(-1).view(np.uint16 if q8 else np.uint32))
+    g = torch.linspace(-1, 1, n, device="cuda")
+    got, = torch.autograd.grad(t1, t, g)
+    scale = 1.0 / 256 if q8 else 1.0
+    w0, w2 = w.double() * scale, w1.detach().double() * scale
+    want = torch.where(w2 > w0, g.double() * w0 / w2.clamp_min(1e-30), g.double())
+    # w0 / (w0 + w), the sum and the two operations rounded once each
+    torch.testing.assert_close(got.double(), want, rtol=4 * 2.0**-24, atol=1e-12)
+    assert (w2 > 0).sum() > 100
 
 
 def test_tsdf_backward_matches_fp64_oracle(tsdf_case):
