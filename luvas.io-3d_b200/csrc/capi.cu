@@ -3033,20 +3033,19 @@ int device_cover(int w, int h, int tw, int th, cudaStream_t s, DeviceCover* out,
     return L3D_OK;
 }
 
-/* resampleArea (gray-image.ts:193-221) of a device source (src_kind as l3d_launch_area), with
- * the coverage tables from the cache and the row-pass buffer from the pool. */
-int area_resample(const void* src, int src_kind, int w, int h, int tw, int th, uint8_t* out,
+/* resampleArea (gray-image.ts:193-221) of a device source, with the coverage tables from the cache
+ * and, for large footprints, a row-pass buffer from the pool. */
+int area_resample(const uint8_t* src, bool rgba, int w, int h, int tw, int th, uint8_t* out,
                   cudaStream_t s) {
     DeviceCover c;
     bool temporary = false;
     int rc = device_cover(w, h, tw, th, s, &c, &temporary);
     if (rc) return rc;
-    float* temp;
-    cudaError_t e = pool_alloc((void**)&temp, (size_t)tw * h * 4, s);
-    if (e == cudaSuccess) {
-        e = l3d_launch_area(src, src_kind, w, h, tw, th, c.cols, c.rows, temp, out, s);
-        cudaFreeAsync(temp, s);
-    }
+    float* temp = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (l3d_area_needs_temp(c.cols, c.rows)) e = pool_alloc((void**)&temp, (size_t)tw * h * 4, s);
+    if (e == cudaSuccess) e = l3d_launch_area(src, rgba, w, h, tw, th, c.cols, c.rows, temp, out, s);
+    if (temp) cudaFreeAsync(temp, s);
     if (temporary) cudaFreeAsync(c.block, s);
     if (e != cudaSuccess) return cuda_fail(e, "area filter launch");
     return L3D_OK;
@@ -3067,7 +3066,7 @@ int l3d_image_rgba_to_gray(const uint8_t* rgba, int32_t width, int32_t height, i
         return L3D_OK;
     }
     /* the area filter reads the RGBA pixels and forms their f32 luma itself */
-    return area_resample(rgba, 2, width, height, target_width, target_height, gray, s);
+    return area_resample(rgba, true, width, height, target_width, target_height, gray, s);
 }
 
 int l3d_image_downsample_rgb(const uint8_t* rgba, int32_t width, int32_t height, int32_t target_width,
@@ -3091,7 +3090,7 @@ int l3d_image_downsample_gray(const uint8_t* gray, int32_t width, int32_t height
                  "gray launch");
         return L3D_OK;
     }
-    return area_resample(gray, 0, width, height, target_width, target_height, out, s);
+    return area_resample(gray, false, width, height, target_width, target_height, out, s);
 }
 
 int l3d_depth_upsample(const float* grid, int32_t grid_width, int32_t grid_height, int32_t width,

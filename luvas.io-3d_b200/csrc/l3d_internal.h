@@ -467,8 +467,10 @@ struct L3dAreaCover {
 
 cudaError_t l3d_launch_gray_blocks(const uint8_t* rgba, int W, int H, int tw, int th, uint8_t* out,
                                    cudaStream_t s);
-/* src_kind: 0 u8 gray, 1 f32, 2 RGBA (its f32 luma) */
-cudaError_t l3d_launch_area(const void* src, int src_kind, int W, int H, int tw, int th,
+/* rgba: an RGBA source (its f32 luma), else u8 gray; temp: tw x H floats where l3d_area_needs_temp, else
+ * NULL */
+bool l3d_area_needs_temp(const L3dAreaCover& cols, const L3dAreaCover& rows);
+cudaError_t l3d_launch_area(const uint8_t* src, bool rgba, int W, int H, int tw, int th,
                             const L3dAreaCover& cols, const L3dAreaCover& rows, float* temp,
                             uint8_t* out, cudaStream_t s);
 cudaError_t l3d_launch_rgb_blocks(const uint8_t* rgba, int W, int H, int tw, int th, uint8_t* out,
