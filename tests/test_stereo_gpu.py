@@ -12,7 +12,7 @@ import oracle
 from helpers import arc_workload, assert_bit_equal
 from luvas3d import (KERNEL_INIT, KERNEL_INIT_COARSE, KERNEL_PACK, KERNEL_PROPAGATE, DenseStereo,
                      L3dError, SolveOptions, StereoOptions, scenes)
-from luvas3d.camera import scale_intrinsics, StereoView
+from luvas3d.camera import Intrinsics, Pose, scale_intrinsics, StereoView
 
 pytestmark = pytest.mark.gpu
 
@@ -247,3 +247,40 @@ def test_errors_are_reported(arc):
     s.destroy()
     with pytest.raises(RuntimeError):
         s.solve(0, SolveOptions([1], 0.5, 5.0))
+
+
+@pytest.mark.parametrize("form", ["camera", "centre 0", "tiny centre", "far source"])
+@pytest.mark.parametrize("n_src,needed", [(1, 1), (3, 2), (4, 3)])
+def test_consistency_filter_forms(form, n_src, needed):
+    """The filter's divisions for calibrations whose operands stay normal numbers, and the general ones
+    (a principal point or a translation beyond their range), on maps with infinite, empty and costly
+    samples: equal to the oracle, bit for bit."""
+    W, H = 131, 75
+    views, imgs, truth, _ = arc_workload(n=5, W=W, H=H, f=W * 0.875)
+    if form in ("centre 0", "tiny centre"):
+        c = 0.0 if form == "centre 0" else 1e-12
+        views = [StereoView(Intrinsics(v.intrinsics.fx, v.intrinsics.fy, c, c), v.pose) for v in views]
+    rng = np.random.default_rng(9)
+    o = oracle.Stereo(W, H, views, imgs, 32)
+    s = gpu_stereo(views, imgs, W, H)
+    for i in range(5):
+        d = (truth[i] * rng.uniform(0.996, 1.004, truth[i].shape)).astype(np.float16)
+        d[::9, ::4] = np.inf
+        d[::5, ::7] = 0
+        m = d.view(np.uint16).astype(np.uint32) | (rng.integers(0, 11, d.shape).astype(np.uint32) << 28 >> 1)
+        o.depths[i][:] = m
+        s.write_depth_map(i, m)
+    src = [1, 3, 0, 4][:n_src]
+    if form == "far source":
+        views = list(views)
+        p = views[src[0]].pose
+        views[src[0]] = StereoView(views[src[0]].intrinsics, Pose(p.R, p.t + np.array([0, 0, 2.0**41])))
+        o, depths = oracle.Stereo(W, H, views, imgs, 32), o.depths
+        s = gpu_stereo(views, imgs, W, H)
+        for i in range(5):
+            o.depths[i][:] = depths[i]
+            s.write_depth_map(i, depths[i])
+    want = o.filter(2, src, needed)
+    assert_bit_equal(s.filtered_map(2, src, needed), want, "filtered")
+    if form == "camera":
+        assert 100 < (want != 0).sum() < W * H
