@@ -46,9 +46,10 @@ __device__ __forceinline__ bool pack_key(double fx, double fy, double fz, unsign
     return true;
 }
 
-/* Slot of the cell (claimed when new), or -1 after setting an error flag. */
-__device__ int claim_key(const L3dCloudTable& t, unsigned long long key, int ix, int iy, int iz, unsigned* used,
+/* Slot of the cell, or -1 after setting an error flag; *fresh: it was claimed now. */
+__device__ int claim_key(const L3dCloudTable& t, unsigned long long key, int ix, int iy, int iz, bool* fresh,
                          int* err) {
+    *fresh = false;
     const unsigned mask = (unsigned)t.capacity - 1u;
     unsigned slot = cell_hash(ix, iy, iz) & mask;
     for (int probe = 0; probe < t.capacity; probe++) {
@@ -57,7 +58,7 @@ __device__ int claim_key(const L3dCloudTable& t, unsigned long long key, int ix,
         if (k == kEmpty) {
             const unsigned long long prev = atomicCAS(t.keys + slot, kEmpty, key);
             if (prev == kEmpty) {
-                atomicAdd(used, 1u);
+                *fresh = true;
                 return (int)slot;
             }
             if (prev == key) return (int)slot;
@@ -68,13 +69,16 @@ __device__ int claim_key(const L3dCloudTable& t, unsigned long long key, int ix,
     return -1;
 }
 __device__ int claim(const L3dCloudTable& t, double cx, double cy, double cz, unsigned* used, int* err) {
+    bool fresh;
     unsigned long long key;
     int ix, iy, iz;
     if (!pack_key(floor(cx), floor(cy), floor(cz), &key, &ix, &iy, &iz)) {
         atomicOr(err, L3D_CLOUD_ERR_RANGE);
         return -1;
     }
-    return claim_key(t, key, ix, iy, iz, used, err);
+    const int slot = claim_key(t, key, ix, iy, iz, &fresh, err);
+    if (fresh) atomicAdd(used, 1u);
+    return slot;
 }
 
 __device__ __forceinline__ void accumulate(const L3dCloudTable& t, int slot, const double* v,
@@ -94,21 +98,22 @@ __device__ void sample_of(const L3dCloudView& v, const double* code, uint32_t va
  * sum: the table sees one set of atomics per cell and warp instead of one per pixel.  The samples meet in
  * shared memory, where every group's first lane sums its own at the same time; passing them along by
  * shuffles ran the groups of a warp (about fifteen) one after the other.  Bound by the table's atomics
- * and FP64 issue: a map of 640x480 takes 19 us, 34 us with shuffles and a row of 32 pixels per warp. */
-constexpr int kMapX = 32, kMapY = 8;  /* pixels per block of 256 threads */
+ * and FP64 issue: a map of 640x480 takes 17.4 us, 34 us with shuffles and a row of 32 pixels per warp.
+ * New cells are counted once per warp (18.8 us with an atomic each on the one counter). */
+constexpr int kMapX = 16, kMapY = 8;  /* pixels per block of 128 threads */
 
-__global__ void __launch_bounds__(256) k_cloud_add_map(const L3dCloudTable t, double cell,
+__global__ void __launch_bounds__(128) k_cloud_add_map(const L3dCloudTable t, double cell,
                                                        const uint32_t* __restrict__ packed, int W, int H,
                                                        const L3dCloudView v, const uint8_t* __restrict__ rgb,
                                                        unsigned* used, int* err) {
     __shared__ double code[64];           /* the decoded values of a 6-bit normal component */
-    __shared__ double samples[256][9];
+    __shared__ double samples[128][9];
     if (threadIdx.x < 64) code[threadIdx.x] = ((double)threadIdx.x / 63.0) * 2.0 - 1.0;
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int across = (W + kMapX - 1) / kMapX, by = blockIdx.x / across, bx = blockIdx.x - by * across;
-    const int x = bx * kMapX + (warp & 3) * 8 + (lane & 7);
-    const int y = by * kMapY + (warp >> 2) * 4 + (lane >> 3);
+    const int x = bx * kMapX + (warp & 1) * 8 + (lane & 7);
+    const int y = by * kMapY + (warp >> 1) * 4 + (lane >> 3);
     const uint32_t value = x < W && y < H ? __ldg(packed + (size_t)y * W + x) : 0u;
     const double d = value ? (double)l3d_f16_to_f32(value & 0xffffu) : 0.0;
     unsigned long long key = 0;
@@ -126,15 +131,21 @@ __global__ void __launch_bounds__(256) k_cloud_add_map(const L3dCloudTable t, do
     if (!valid) return;
     const unsigned group = __match_any_sync(active, key);
     __syncwarp(active);
-    if (lane != __ffs(group) - 1) return;
+    /* the claim's memory round trips first: the sum is ready before they are */
+    const bool leads = lane == __ffs(group) - 1;
+    bool fresh = false;
+    int slot = -1;
+    if (leads) slot = claim_key(t, key, ix, iy, iz, &fresh, err);
+    const unsigned claimed = __ballot_sync(active, fresh);
+    if (claimed && lane == __ffs(active) - 1) atomicAdd(used, (unsigned)__popc(claimed));
+    if (slot < 0) return;
     double s[9] = {};
     for (unsigned m = group; m; m &= m - 1u) {
         const double* q = samples[(threadIdx.x & ~31u) + __ffs(m) - 1];
 #pragma unroll
         for (int k = 0; k < 9; k++) s[k] += q[k];
     }
-    const int slot = claim_key(t, key, ix, iy, iz, used, err);
-    if (slot >= 0) accumulate(t, slot, s, (unsigned)__popc(group));
+    accumulate(t, slot, s, (unsigned)__popc(group));
 }
 
 /* The world sample of one valid pixel (depth d > 0): position, normal, thumbnail colour. */
@@ -401,7 +412,7 @@ cudaError_t l3d_launch_cloud_add_map(const L3dCloudTable& t, double cell, const 
                                      unsigned* used, int* err, cudaStream_t stream) {
     if ((long long)W * H == 0) return cudaSuccess;
     const long long blocks = (long long)((W + kMapX - 1) / kMapX) * ((H + kMapY - 1) / kMapY);
-    k_cloud_add_map<<<(unsigned)blocks, 256, 0, stream>>>(t, cell, packed, W, H, v, rgb, used, err);
+    k_cloud_add_map<<<(unsigned)blocks, 128, 0, stream>>>(t, cell, packed, W, H, v, rgb, used, err);
     return cudaGetLastError();
 }
 
