@@ -553,17 +553,22 @@ __global__ void k_visible_depth(const L3dTsdfGrid g, const L3dTsdfView* __restri
     mask[t] = brick_behind_depths<false>(g, views[vi], tiles, bx, by, bz) ? 0 : brick_visible(g, views[vi], bx, by, bz);
 }
 
-/* The kept bricks of one view, eight lanes per brick: list[0] counts them (zeroed before the launch),
- * list[1..] receives their indices in any order. */
+/* The kept bricks of one view, a thread per brick, or eight (LANES): list[0] counts them (zeroed before the
+ * launch), list[1..] receives their indices in any order.  Eight lanes shorten the walk over a brick's tiles,
+ * one makes an eighth of the frustum tests' FP64 instructions: a view of 640x480 and all its launches take
+ * 24.8 against 41.7 us at 3472 bricks, 25.6 against 29.9 at 110592, but 32.4 against 31.1 at 175616 and
+ * 39.8 against 32.4 at 262144. */
+constexpr long long LANES_BRICKS = 1 << 17;
+template <bool LANES>
 __global__ void __launch_bounds__(128) k_visible_one_list(const L3dTsdfGrid g, const L3dTsdfView v,
                                                           const int32_t* __restrict__ coords,
                                                           const float* __restrict__ tiles, int32_t* __restrict__ list) {
-    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> (LANES ? 3 : 0);
     const long long b = t < g.bricks ? t : g.bricks - 1;  /* every lane takes part */
     int bx, by, bz;
     brick_coords(g, coords, b, &bx, &by, &bz);
-    const bool behind = brick_behind_depths<true>(g, v, tiles, bx, by, bz);
-    if (behind || t >= g.bricks || (threadIdx.x & 7) != 0 || !brick_visible(g, v, bx, by, bz)) return;
+    const bool behind = brick_behind_depths<LANES>(g, v, tiles, bx, by, bz);
+    if (behind || t >= g.bricks || (LANES && (threadIdx.x & 7) != 0) || !brick_visible(g, v, bx, by, bz)) return;
     list[1 + atomicAdd(list, 1)] = (int32_t)b;
 }
 
@@ -1246,7 +1251,10 @@ cudaError_t l3d_launch_tsdf_view(const L3dTsdfGrid& g, const L3dTsdfView& v, con
         k_depth_tiles_one<<<(unsigned)((nt * 8 + 127) / 128), 128, 0, stream>>>(vt, depth, prior, tiles, list);
         cudaError_t e;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_visible_one_list<<<(unsigned)((g.bricks * 8 + 127) / 128), 128, 0, stream>>>(g, vt, coords, tiles, list);
+        if (g.bricks <= LANES_BRICKS)
+            k_visible_one_list<true><<<(unsigned)((g.bricks * 8 + 127) / 128), 128, 0, stream>>>(g, vt, coords, tiles, list);
+        else
+            k_visible_one_list<false><<<(unsigned)((g.bricks + 127) / 128), 128, 0, stream>>>(g, vt, coords, tiles, list);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         const unsigned blocks = (unsigned)std::min<long long>(148 * 8, (g.bricks * 128 + 255) / 256);
         if (vec4_ok(g)) {

@@ -329,3 +329,19 @@ def test_range_limits_and_remainders_bit_exact(scene, dims, mu, q8):
         t, w = g.read()
         assert np.all(t == 1.0) and np.all(w == 0)
     assert (o.weight > 0).sum() > 1000
+
+
+@pytest.mark.parametrize("dims", [(512, 512, 256), (512, 512, 264)])
+def test_view_list_of_many_bricks_equals_sweep(scene, dims):
+    """Grids on both sides of the brick count up to which the one-view cull takes eight lanes per brick
+    (131072 and 135168 bricks): the same volume as the sweep's own cull."""
+    views, maps = scene
+    a, b = (TsdfVolume(120, 90, 0.008, (-2.0, -2.0, -1.0), dense=dims, truncation=0.03, weight_q8=True)
+            for _ in range(2))
+    for i in (0, 3):
+        a.integrate(gpu_view(views[i]), depth=maps[i])
+    b.integrate_many([gpu_view(views[i]) for i in (0, 3)], depths=np.stack([maps[0], maps[3]]))
+    (ta, wa), (tb, wb) = a.read(), b.read()
+    assert_bit_equal(ta, tb, "tsdf")
+    assert_bit_equal(wa, wb, "weight")
+    assert (wa > 0).sum() > 5000
