@@ -22,14 +22,15 @@
  * sums in face order.  Each vertex gathers its faces (a CSR of vertex -> faces, each list sorted
  * by face index) and sums them in that order, so the f32 sums round exactly as the reference's.
  *
- * Components (mesh.ts:37-87): union-find over the faces' edges (one root is hooked onto the other with a
- * compare-and-swap, paths are shortened on the way); the kept faces keep their order
- * and vertices are renumbered in order of first use, as the reference's union-find pass does.
+ * Components (mesh.ts:37-87): union-find over the faces' edges (l3d_labels.h: one root is hooked onto the
+ * other with a compare-and-swap, paths are shortened on the way); the kept faces keep their order and
+ * vertices are renumbered in order of first use, as the reference's union-find pass does.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "l3d_internal.h"
+#include "l3d_labels.h"
 
 namespace {
 
@@ -497,61 +498,36 @@ __global__ void k_cc_init(long long vertices, uint32_t* label) {
     if (v < vertices) label[v] = (uint32_t)v;
 }
 
-constexpr int kGuard = 1 << 24;  /* steps along labels, each to a vertex of lower rank */
-
-/* The root of v; every vertex passed is pointed at its successor's successor.  Such a store can overwrite
- * a shorter path another thread stored, never a root's hook (a root is only written by the
- * compare-and-swap that ends its being one). */
-__device__ __forceinline__ uint32_t root_of(uint32_t* label, uint32_t v, int* err) {
-    uint32_t p = __ldcg(label + v);
-    for (int guard = 0; p != v; guard++) {
-        const uint32_t g = __ldcg(label + p);
-        if (g == p) break;
-        if (guard >= kGuard) {
-            *err = 1;
-            break;
-        }
-        __stcg(label + v, g);
-        v = p;
-        p = g;
+/* Labels in global memory.  Other threads change them meanwhile, so every access is one relaxed operation
+ * that the compiler neither repeats nor merges with another. */
+struct GlobalLabels {
+    uint32_t* label;
+    __device__ __forceinline__ uint32_t load(uint32_t v) const {
+        uint32_t l;
+        asm volatile("ld.relaxed.gpu.u32 %0, [%1];" : "=r"(l) : "l"(label + v) : "memory");
+        return l;
     }
-    return p;
-}
-
-/* A vertex's rank among roots: a bijection, so ranks are distinct, and mixed, so that linking a mesh's
- * vertices in their scan order does not build long chains (linked by index, 74 thousand faces took 93
- * us). */
-__device__ __forceinline__ uint32_t cc_rank(uint32_t v) {
-    v ^= v >> 15;
-    v *= 0x2c1b3c6du;
-    v ^= v >> 12;
-    return v * 0x297a2d39u;
-}
-
-/* Joins the components of a and b: the root of higher rank onto the other. */
-__device__ __forceinline__ void unite(uint32_t* label, uint32_t a, uint32_t b, int* err) {
-    for (int guard = 0; guard < kGuard; guard++) {
-        a = root_of(label, a, err);
-        b = root_of(label, b, err);
-        if (a == b) return;
-        const bool a_up = cc_rank(a) > cc_rank(b);
-        const uint32_t hi = a_up ? a : b, lo = a_up ? b : a;
-        if (atomicCAS(label + hi, hi, lo) == hi) return;
+    __device__ __forceinline__ void store(uint32_t v, uint32_t l) const {
+        asm volatile("st.relaxed.gpu.u32 [%0], %1;" : : "l"(label + v), "r"(l) : "memory");
     }
-    *err = 1;
-}
+    __device__ __forceinline__ bool swap(uint32_t v, uint32_t from, uint32_t to) const {
+        return atomicCAS(label + v, from, to) == from;
+    }
+};
 
 __global__ void k_cc_unite(const uint32_t* idx, long long faces, uint32_t* label, int* err) {
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= faces) return;
     const uint32_t a = idx[f * 3], b = idx[f * 3 + 1], c = idx[f * 3 + 2];
-    unite(label, a, b, err);
-    unite(label, b, c, err);
+    GlobalLabels m = {label};
+    l3d_label_unite(m, a, b, err);
+    l3d_label_unite(m, b, c, err);
 }
 
 __global__ void k_cc_flatten(long long vertices, uint32_t* label, int* err) {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < vertices) __stcg(label + v, root_of(label, (uint32_t)v, err));
+    GlobalLabels m = {label};
+    if (v < vertices) l3d_label_flatten(m, (uint32_t)v, err);
 }
 
 /* Faces per component; the lanes of a warp that share one add once. */
