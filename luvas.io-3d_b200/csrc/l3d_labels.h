@@ -11,6 +11,8 @@
 
 #include <stdint.h>
 
+#include "l3d_fmath.h"
+
 #ifdef __CUDACC__
 #define L3D_LABELS __device__ __forceinline__
 #else
@@ -19,15 +21,11 @@
 
 constexpr int kLabelGuard = 1 << 24;  /* steps along labels, each to a vertex of lower rank */
 
-/* A vertex's rank among roots: a bijection, so ranks are distinct, and mixed, so that linking a mesh's
- * vertices in their scan order does not build long chains (linked by index, 74 thousand faces took 93
- * us). */
-L3D_LABELS uint32_t l3d_label_rank(uint32_t v) {
-    v ^= v >> 15;
-    v *= 0x2c1b3c6du;
-    v ^= v >> 12;
-    return v * 0x297a2d39u;
-}
+/* A vertex's rank among roots: the random numbers' hash (l3d_fmath.h).  It is a bijection (an affine map
+ * with an odd factor, a xorshift by an amount that the top bits, which it keeps, give, a product with an
+ * odd number, another xorshift), so ranks are distinct; and it mixes, so that linking a mesh's vertices
+ * in their scan order does not build long chains (linked by index, 74 thousand faces took 93 us). */
+L3D_HD uint32_t l3d_label_rank(uint32_t v) { return l3d_pcg(v); }
 
 /* The root of v while components are joined; every vertex passed is pointed at its successor's successor.
  * Such a store can overwrite a shorter path that another thread stored: the vertex still leads to its
