@@ -208,7 +208,7 @@ struct HostOut {
 };
 
 /* Copies up to kMaxOuts device arrays into host ones in the order of stream `s`, the last piece waited for.  Pageable
- * targets go through the courier's buffers, one being filled while the other is copied out; pinned ones
+ * targets go through the courier's buffers, one being filled while the other is copied out; the others
  * are copied directly. */
 cudaError_t deliver(Courier* c, cudaStream_t s, const HostOut* outs, int n) {
     cudaError_t e;
@@ -234,13 +234,16 @@ cudaError_t deliver(Courier* c, cudaStream_t s, const HostOut* outs, int n) {
     };
     for (int i = 0; i < n; i++) {
         if (!outs[i].host || !outs[i].bytes) continue;
+        /* memory that CUDA knows (pinned, managed, and a device's, which the host must not touch) goes to the
+         * runtime's copy, which takes it or refuses it with a status */
         cudaPointerAttributes attr;
-        if (cudaPointerGetAttributes(&attr, outs[i].host) == cudaSuccess && attr.type == cudaMemoryTypeHost) {
+        const bool known = cudaPointerGetAttributes(&attr, outs[i].host) == cudaSuccess;
+        if (!known) cudaGetLastError();
+        if (known && attr.type != cudaMemoryTypeUnregistered) {
             if ((e = cudaMemcpyAsync(outs[i].host, outs[i].dev, outs[i].bytes, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
                 return e;
             continue;
         }
-        cudaGetLastError();
         for (size_t at = 0; at < outs[i].bytes;) {
             const size_t take = std::min(outs[i].bytes - at, Courier::kBytes - used);
             if ((e = cudaMemcpyAsync(c->buffer[cur] + used, (const char*)outs[i].dev + at, take,
