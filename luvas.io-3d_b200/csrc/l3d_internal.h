@@ -87,8 +87,8 @@ bool l3d_tsdf_grid_of(const l3d_tsdf_desc* d, bool pool_coords_given, L3dTsdfGri
 L3dTsdfView l3d_tsdf_view_of(const l3d_integration_view& v);
 
 /* Whether the numbers of these views' integration stay ordinary (tsdf.cu): |camera coordinates| < 2^50,
- * mu in [2^-60, 2^60], map sides at most 2^22.  The kernels over lists of kept bricks rely on it; what
- * is not ordinary goes through the general ones. */
+ * mu in [2^-60, 2^60], map sides at most 2^22 and fewer than 2^31 pixels.  The kernels over lists of kept
+ * bricks rely on it; what is not ordinary goes through the general ones. */
 bool l3d_tsdf_ordinary(const L3dTsdfGrid& g, const L3dTsdfView* views, int n);
 
 /* ---- launchers (stereo.cu / stereo_fast.cu / tsdf.cu); each returns cudaGetLastError() ---- */

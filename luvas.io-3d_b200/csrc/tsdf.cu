@@ -38,6 +38,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include <cuda_fp16.h>
 
@@ -134,10 +135,14 @@ __device__ __forceinline__ bool observe(const L3dTsdfGrid& g, const L3dTsdfView&
  * same values without the general division's branches and without the conversion pipe, which a voxel
  * and view otherwise enters five times (reciprocal, two roundings, two conversions) at a quarter of
  * the FMA rate or less.  The sweep of 24 views into 512^3: 426 -> 322 us
- * (270 us with bricks handed out, see k_integrate_many_list). */
+ * (270 us with bricks handed out, see k_integrate_many_list).  An ordinary map has fewer than 2^31
+ * pixels; the indices of any other (17 GB and more with its FP32 depths) have 64 bits. */
+template <bool ORD>
+using PixelIndex = typename std::conditional<ORD, int, long long>::type;
+
 template <bool ORD>
 __device__ __forceinline__ bool lut_pixel(const L3dTsdfView& v, float wx, float wy, float wz,
-                                          float3* cam_out, int* pix) {
+                                          float3* cam_out, PixelIndex<ORD>* pix) {
     const float* R = v.R;
     float3 cam = make_float3(fmaf(R[2], wz, fmaf(R[1], wy, fmaf(R[0], wx, v.t[0]))),
                              fmaf(R[5], wz, fmaf(R[4], wy, fmaf(R[3], wx, v.t[1]))),
@@ -155,15 +160,15 @@ __device__ __forceinline__ bool lut_pixel(const L3dTsdfView& v, float wx, float 
     float rx = rintf(fmaf(v.k[0] * cam.x, iz, v.k[2]));
     float ry = rintf(fmaf(v.k[1] * cam.y, iz, v.k[3]));
     if (!(rx >= 0.0f && ry >= 0.0f && rx < (float)v.W && ry < (float)v.H)) return false;
-    *pix = (int)ry * v.W + (int)rx;
+    *pix = (PixelIndex<ORD>)(int)ry * v.W + (int)rx;
     return true;
 }
 
 template <bool ORD>
 __device__ __forceinline__ bool lut_observe(const L3dTsdfGrid& g, const L3dTsdfView& v,
                                             const float* __restrict__ prior,
-                                            const float4* __restrict__ normals, float3 cam, int i,
-                                            uint32_t packed, float* obs, float* wout) {
+                                            const float4* __restrict__ normals, float3 cam,
+                                            PixelIndex<ORD> i, uint32_t packed, float* obs, float* wout) {
     float d = __half2float(__ushort_as_half((unsigned short)(packed & 0xffffu)));
     const bool stereo = d > 0.0f;
     if (!stereo) d = prior ? __ldg(prior + i) : 0.0f;
@@ -605,7 +610,7 @@ __device__ __forceinline__ void integrate_quad(const L3dTsdfGrid& g, const L3dTs
         const float wz = fmaf((float)gz + 0.5f, g.voxel, g.origin[2]);
         const float* pr = v.has_prior ? prior : nullptr;
         float3 cam[VEC];
-        int pix[VEC];
+        PixelIndex<ORD> pix[VEC];
         uint32_t packed[VEC];
 #pragma unroll
         for (int j = 0; j < VEC; j++)
@@ -760,7 +765,7 @@ __device__ __forceinline__ void sweep_quad(const L3dTsdfGrid& g, const L3dTsdfVi
         const uint32_t* depth = depths[vi];
         const float* prior = v.has_prior ? priors + v.prior_off : nullptr;
         float3 cam[VEC];
-        int pix[VEC];
+        PixelIndex<ORD> pix[VEC];
         bool in[VEC];
         uint32_t packed[VEC];
 #pragma unroll
@@ -909,7 +914,7 @@ __global__ void __launch_bounds__(256) k_count_updates(const L3dTsdfGrid g,
 #pragma unroll
             for (int j = 0; j < VEC; j++) {
                 float3 cam;
-                int pix;
+                PixelIndex<false> pix;
                 float obs, w;
                 if (lut_pixel<false>(v, fmaf((float)(gx + j) + 0.5f, g.voxel, g.origin[0]), wy, wz, &cam, &pix) &&
                     lut_observe<false>(g, v, prior, normals, cam, pix, __ldg(depths[vi] + pix), &obs, &w))
@@ -939,8 +944,9 @@ __device__ __forceinline__ bool observe_diff(const L3dTsdfGrid& g, const L3dTsdf
                                              const float* __restrict__ depthf,
                                              const float* __restrict__ prior,
                                              const float4* __restrict__ normals, float3 cam, uint32_t packed,
-                                             int* pix, float* obs, float* wout, float* dobs, float* dw) {
-    const int i = *pix;
+                                             PixelIndex<ORD>* pix, float* obs, float* wout, float* dobs,
+                                             float* dw) {
+    const PixelIndex<ORD> i = *pix;
     const bool stereo = __half2float(__ushort_as_half((unsigned short)(packed & 0xffffu))) > 0.0f;
     const float d = stereo ? __ldg(depthf + i) : (prior ? __ldg(prior + i) : 0.0f);
     if (!(d > 0.0f)) return false;
@@ -977,7 +983,7 @@ __device__ __forceinline__ bool observe_diff(const L3dTsdfGrid& g, const L3dTsdf
 template <int VEC, bool ORD>
 __device__ __forceinline__ unsigned quad_pixels(const L3dTsdfGrid& g, const L3dTsdfView& v,
                                                 const uint32_t* __restrict__ depth, int gx, int gy, int gz,
-                                                float3* cam, int* pix, uint32_t* packed) {
+                                                float3* cam, PixelIndex<ORD>* pix, uint32_t* packed) {
     const float wy = fmaf((float)gy + 0.5f, g.voxel, g.origin[1]);
     const float wz = fmaf((float)gz + 0.5f, g.voxel, g.origin[2]);
     unsigned in = 0u;
@@ -1055,7 +1061,7 @@ __global__ void __launch_bounds__(256) k_integrate_depth(const L3dTsdfGrid g, co
     else load_quad<VEC>((const float*)weight_in + idx, wf);
     if (mask[brick]) {
         float3 cam[VEC];
-        int pix[VEC];
+        PixelIndex<ORD> pix[VEC];
         uint32_t packed[VEC];
         const unsigned in = quad_pixels<VEC, ORD>(g, v, depth, gx, gy, gz, cam, pix, packed);
 #pragma unroll
@@ -1103,7 +1109,7 @@ __global__ void __launch_bounds__(256) k_integrate_depth_grad(
     if (!Q8 && gW) load_quad<VEC>(gW + idx, gw);
     if (mask[brick]) {
         float3 cam[VEC];
-        int pix[VEC];
+        PixelIndex<ORD> pix[VEC];
         uint32_t packed[VEC];
         const unsigned in = quad_pixels<VEC, ORD>(g, v, depth, gx, gy, gz, cam, pix, packed);
 #pragma unroll
@@ -1168,7 +1174,7 @@ bool l3d_tsdf_ordinary(const L3dTsdfGrid& g, const L3dTsdfView* views, int n) {
         reach[i] = std::fabs(g.origin_d[i]) + (g.dense ? (double)g.dims[i] + 8.0 : 0x1p35) * g.voxel_d;
     for (int k = 0; k < n; k++) {
         const L3dTsdfView& v = views[k];
-        if (v.W > 1 << 22 || v.H > 1 << 22) return false;
+        if (v.W > 1 << 22 || v.H > 1 << 22 || (long long)v.W * v.H >= 1ll << 31) return false;
         for (int r = 0; r < 3; r++) {
             double bound = std::fabs((double)v.t[r]);
             for (int i = 0; i < 3; i++) bound += std::fabs((double)v.R[r * 3 + i]) * reach[i];
