@@ -451,11 +451,12 @@ __global__ void __launch_bounds__(128) k_init_coarse(const L3dParams p, const L3
  * in both).  The dense 11 x 11 window, whose pairs a thread alone keeps in local memory, went from
  * 53.7 to 9.7 ms at 640x480 (4 sources, 2 iterations). */
 constexpr int kPropagateBlocks = 6;
+constexpr int kGridRows = 65535;  /* the most blocks a launch has along y: taller images go on along z */
 template <int N, int DIL>
 __global__ void __launch_bounds__(128, kPropagateBlocks) k_propagate(const L3dParams p, const L3dStereoDev d) {
     __shared__ float2 windows[N * N * 16];
     const int warp = threadIdx.x >> 5, sub = (threadIdx.x >> 3) & 3, cand = threadIdx.x & 7;
-    int y = blockIdx.y * 2 + (sub >> 1);
+    int y = (blockIdx.z * kGridRows + blockIdx.y) * 2 + (sub >> 1);
     int x = (blockIdx.x * 8 + warp * 2 + (sub & 1)) * 2 + (int)((y + p.phase) & 1u);
     const bool inside = x < p.W && y < p.H;
     if (!__any_sync(0xffffffffu, inside)) return;
@@ -611,8 +612,9 @@ cudaError_t launch_win(int kernel, const L3dParams& p, const L3dStereoDev& d, cu
             break;
         }
         case L3D_K_PROPAGATE: {
-            const int half = (p.W + 1) / 2;
-            k_propagate<N, DIL><<<dim3((half + 7) / 8, (p.H + 1) / 2), 128, 0, stream>>>(p, d);
+            const int half = (p.W + 1) / 2, rows = (p.H + 1) / 2;
+            const dim3 grid((half + 7) / 8, rows < kGridRows ? rows : kGridRows, (rows + kGridRows - 1) / kGridRows);
+            k_propagate<N, DIL><<<grid, 128, 0, stream>>>(p, d);
             break;
         }
         default:
