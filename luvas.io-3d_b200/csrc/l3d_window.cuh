@@ -47,8 +47,10 @@ __device__ __forceinline__ L3dPlace l3d_window_place(const float* h, float px, f
     const float mz = fmaf(fabsf(h[6]), ax, fmaf(fabsf(h[7]), ay, fabsf(h[8])));
     const float unit = 0x1p-20f * l3d_rcp_approx(zmin);
     const float su = unit * fmaf(wmax, mz, mx), sv = unit * fmaf(hmax, mz, my);
-    if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv && umax <= wmax - su &&
-        vmax <= hmax - sv)
+    /* strictly below the last texel, whose footprint has no right or lower neighbour: su is 0 where a row of
+     * H is, and the window of such an H lies on one texel of an image one pixel wide */
+    if (zmin > fmaf(0x1p-20f, mz, 1e-6f) && zmax < 0x1p120f && umin >= su && vmin >= sv && umax < wmax - su &&
+        vmax < hmax - sv)
         return L3D_INSIDE;
     if (zmin <= 1e-6f || umin < -su || vmin < -sv || umax > wmax + su || vmax > hmax + sv) return L3D_OUTSIDE;
     return L3D_GRAZES;
