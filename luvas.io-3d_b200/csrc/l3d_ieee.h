@@ -8,8 +8,8 @@
  *   reciprocal  one Newton step on the hardware approximation y (error at most one ulp):
  *               y + y (1 - x y), both operations fused.  Markstein ("Computation of elementary
  *               functions on the IBM RISC System/6000 processor", IBM J. R&D 34, 1990) shows that
- *               the step rounds correctly but for a divisor of all-ones mantissa; compared with
- *               1.0f / x over every mantissa at every seventh exponent it never differed.
+ *               the step rounds correctly but for a divisor of all-ones mantissa; those come out
+ *               right too: over every float of the range it equals 1.0f / x (tests/test_ieee_gpu.py).
  *   quotient    his theorem for a / b from a correctly rounded reciprocal: q = a y, then
  *               q + y (a - b q), the remainder exact.
  */
