@@ -816,11 +816,14 @@ __global__ void __launch_bounds__(256, 4) k_integrate_many(const L3dTsdfGrid g,
 
 /* The sweep over the bricks some view keeps: list holds them in ascending order
  * (l3d_launch_tsdf_brick_list), prefix[b] is the number of kept bricks below brick b, so the
- * kept bricks of [b_begin, b_end) are list[prefix[b_begin] .. prefix[b_end]).  A warp takes the next
- * brick from *next (zeroed before the launch) until none is left: bricks cost as much as views keep
- * them, and a fixed share per warp leaves warps idle at the end (24 views into
- * 512^3: 322 us, handed out 270 us).  Each quad is still one
- * thread's, so results equal k_integrate_many's. */
+ * kept bricks of [b_begin, b_end) are list[prefix[b_begin] .. prefix[b_end]).  A
+ * warp's pass takes 32 quads of a brick.  Every warp starts with a share of passes by its number and takes
+ * the next ones from *next (zeroed before the launch, see there) until none is left: bricks cost as much
+ * as views keep them, and a fixed share for each warp leaves warps idle at the end (24 views into 512^3: 322
+ * us, handed out 270 us).  A share is at most a brick, for few atomics, and an eighth of what there is for
+ * each warp, at least a pass: whole bricks left most of the chip waiting for warps that walked their 4
+ * or 16 passes alone where few bricks are kept (host call, 24 views of 320x240: 101^3 278 -> 147 us, 256^3
+ * 236 -> 171).  Each quad is still one thread's, so results equal k_integrate_many's. */
 template <int VEC, bool Q8>
 __global__ void __launch_bounds__(256, 4) k_integrate_many_list(const L3dTsdfGrid g,
                                                              const L3dTsdfView* __restrict__ views,
@@ -847,18 +850,24 @@ __global__ void __launch_bounds__(256, 4) k_integrate_many_list(const L3dTsdfGri
         for (int k = threadIdx.x; k < words; k += blockDim.x) dst[k] = __ldg(src + k);
         __syncthreads();
     }
-    const uint32_t first = __ldg(prefix + b_begin), n = __ldg(prefix + b_end) - first;
+    constexpr uint32_t PASSES = PER / 32;  /* of a warp over a brick */
+    const uint32_t first = __ldg(prefix + b_begin), passes = (__ldg(prefix + b_end) - first) * PASSES;
     const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t share = min(max(passes / (warps * 8u), 1u), PASSES);
+    uint32_t at = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     for (;;) {
-        uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(next, 1u);
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i >= n) return;
-        const long long b = __ldg(list + first + i);
-        for (int k = lane; k < PER; k += 32)
+        const uint32_t begin = at * share, end = min(begin + share, passes);
+        for (uint32_t i = begin; i < end; i++) {
+            const long long b = __ldg(list + first + i / PASSES);
             sweep_quad<VEC, Q8, true>(g, sv, n_views, coords, mask, depths, priors, normals, tsdf, weight,
-                                      b * PER + k);
-        __syncwarp();
+                                      b * PER + (i % PASSES) * 32u + lane);
+            __syncwarp();
+        }
+        if (end >= passes || warps * share >= passes) return;
+        if (lane == 0) at = atomicAdd(next, 1u);
+        at = warps + __shfl_sync(0xffffffffu, at, 0);
+        if (at * share >= passes) return;
     }
 }
 static_assert(sizeof(L3dTsdfView) % 8 == 0, "the view table is copied in 8-byte words");
@@ -1375,7 +1384,7 @@ cudaError_t l3d_launch_tsdf_many_list(const L3dTsdfGrid& g, const L3dTsdfView* v
     q_end = q_end < quad_count(g, vec) ? q_end : quad_count(g, vec);
     if (q_end <= q_begin || n_views == 0) return cudaSuccess;
     const long long b0 = q_begin / per, b1 = (q_end + per - 1) / per;
-    /* four resident blocks per SM, bricks handed out as warps ask */
+    /* four resident blocks per SM, passes handed out as warps ask */
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
@@ -1387,8 +1396,11 @@ cudaError_t l3d_launch_tsdf_many_list(const L3dTsdfGrid& g, const L3dTsdfView* v
     if (smem > 48 * 1024 || !ordinary)
         return l3d_launch_tsdf_many_range(g, views_dev, n_views, coords, mask, depth_ptrs_dev, priors,
                                           normals, tsdf, weight, q8, q_begin, q_end, stream);
-    const cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return e;
+    /* where even all bricks kept are a pass or less for each warp, none of them asks */
+    if ((b1 - b0) * (per / 32) > (long long)blocks * 8) {
+        const cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
+        if (e != cudaSuccess) return e;
+    }
     if (vec == 4) {
         if (q8) k_integrate_many_list<4, true><<<blocks, 256, smem, stream>>>(g, views_dev, n_views, coords, mask, depth_ptrs_dev, priors, normals, tsdf, weight, prefix, list, next, b0, b1);
         else k_integrate_many_list<4, false><<<blocks, 256, smem, stream>>>(g, views_dev, n_views, coords, mask, depth_ptrs_dev, priors, normals, tsdf, weight, prefix, list, next, b0, b1);
