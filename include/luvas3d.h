@@ -259,8 +259,9 @@ int64_t l3d_stereo_launches(const l3d_stereo* s);
  * weights instead of the hardware filter.  All variants compute the same algorithm; fast-form
  * results differ only by the texture unit's 8-bit filter weights on the rows it filters.  The
  * exact form and compensated sums take 6 rows (the exact form always gathers).  + 8 and + 32
- * (fast form, 6 rows) once chose a lane mapping and a place for the reference window; they are
- * still accepted and reported, and select nothing: the kernels pick both by the launch's size. */
+ * once chose a lane mapping and a place for the reference window; they are accepted where they were
+ * then (+ 32: fast form, U8, F16 or F32 storage, 6 rows) and reported, and select nothing: the window is
+ * always in shared memory, and the lanes follow the launch's size. */
 int l3d_stereo_set_variant(l3d_stereo* s, int32_t variant);
 int32_t l3d_stereo_variant(const l3d_stereo* s);
 

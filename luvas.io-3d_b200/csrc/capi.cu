@@ -1495,21 +1495,22 @@ int l3d_stereo_set_variant(l3d_stereo* s, int32_t variant) {
     if (!s) return fail(L3D_EINVAL, "NULL handle");
     if (!batched(s)) return fail(L3D_ESTATE, "variants select fast- and exact-form kernels");
     const int rows = variant & 7, rest = variant & ~63;
+    /* 32 once put the reference window in shared memory, where it always is now: it selects nothing and is
+     * taken where it was then */
     const bool gather = (variant & 16) != 0, shared_window = (variant & 32) != 0;
     if (rest || !(rows == 6 || rows == 4 || rows == 3 || rows == 2))
-        return fail(L3D_EINVAL, "variant %d: texture rows must be 6, 4, 3 or 2 (+8 for quads, +16 "
-                                "for gathers, +32 for a shared-memory window)", variant);
+        return fail(L3D_EINVAL, "variant %d: texture rows must be 6, 4, 3 or 2 (+16 for gathers; "
+                                "+8 and +32 select nothing)", variant);
     if (rows != 6 && (s->opts.form == L3D_FORM_EXACT || s->opts.compensated || gather || shared_window))
-        return fail(L3D_EINVAL, "variant %d: the exact form, compensated sums, gathers and the "
-                                "shared-memory window sample all six rows through the texture unit",
+        return fail(L3D_EINVAL, "variant %d: the exact form, compensated sums, gathers and +32 "
+                                "go with all six rows through the texture unit",
                     variant);
     if (gather && (s->opts.form != L3D_FORM_FAST || s->opts.storage == L3D_DTYPE_BF16))
         return fail(L3D_EINVAL, "variant %d: gathers with exact weights are a fast-form option for "
                                 "texture storage (U8, F16, F32); the exact form always gathers", variant);
     if (shared_window && (s->opts.form != L3D_FORM_FAST || s->opts.storage == L3D_DTYPE_BF16))
-        return fail(L3D_EINVAL, "variant %d: the shared-memory window is a fast-form option for "
-                                "texture storage (U8, F16, F32); the exact form always keeps its "
-                                "window in shared memory", variant);
+        return fail(L3D_EINVAL, "variant %d: +32 is taken by the fast form with texture storage (U8, F16, "
+                                "F32) only, and selects nothing there", variant);
     s->variant = variant;
     return L3D_OK;
 }

@@ -356,9 +356,9 @@ __device__ __forceinline__ float hyp_cost(const E& e, const L3dFastView& v, cons
 }
 
 /* One pixel's reference window in shared memory: 36 pairs of window values, pair i at
- * win[i * STRIDE].  The propagate kernel keeps a pixel's pairs together (STRIDE 1: the eight lanes
- * of a pixel read the same pair, a broadcast); the kernels with one thread per pixel keep a column
- * per thread (STRIDE 128: consecutive threads read consecutive pairs).  The exact evaluator's pairs
+ * win[i * STRIDE].  k_fast_propagate_lanes keeps a pixel's pairs together (STRIDE 1: the eight lanes
+ * of a pixel read the same pair, a broadcast); the kernels with one thread per pixel, k_fast_propagate
+ * among them, keep a column per thread (STRIDE 128: consecutive threads read consecutive pairs).  The exact evaluator's pairs
  * are (w, r), the fast evaluator's (w, w (r - c)), c the centre pixel. */
 constexpr int XBLOCK = 128;
 
@@ -1007,8 +1007,8 @@ cudaError_t l3d_launch_make_pairs(const void* img, int storage, int W, int H, ui
 
 /* variant = texture rows (6, 4, 3, 2; the exact evaluator, compensated sums and gathers take 6
  * only) + 16 x texture gathers with exact weights (fast evaluator, F16/F32/U8).  The quad (8) and
- * shared-window (32) bits of earlier kernels select nothing any more: the propagate kernel always
- * keeps the window in shared memory and a pixel's candidates in quads. */
+ * shared-window (32) bits of earlier kernels select nothing any more: both propagate kernels keep
+ * the window in shared memory, and the thread-per-pixel one always maps quads to 2 x 2 pixels. */
 cudaError_t l3d_launch_fast(int kernel, const L3dFastDev& d, int iteration, int phase, int variant,
                             cudaStream_t stream) {
     if (d.total_tiles <= 0) return cudaSuccess;

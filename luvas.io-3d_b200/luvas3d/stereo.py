@@ -295,7 +295,7 @@ class DenseStereo:
     @property
     def variant(self) -> int:
         """Batched-form kernel variant: texture-sampled window rows + 16 x texture gathers with exact
-        weights (+ 8 and + 32 are accepted and select nothing)."""
+        weights (+ 8 and + 32 are accepted where they once chose, and select nothing)."""
         return int(self._lib.l3d_stereo_variant(self._h()))
 
     @variant.setter
