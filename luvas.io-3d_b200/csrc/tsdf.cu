@@ -814,12 +814,18 @@ __global__ void __launch_bounds__(256, 4) k_integrate_many(const L3dTsdfGrid g,
     sweep_quad<VEC, Q8, false>(g, views, n_views, coords, mask, depths, priors, normals, tsdf, weight, q);
 }
 
+/* Passes per warp up to which the sweep's warps stride through them by their numbers: asking costs a round
+ * trip each and the counter's clearing a node of the stream (66^3, 5 views of 320x240: 86.7 us with
+ * asking, 84.4 without), and balances nothing yet; at 8 rounds it would (256^3, 24 views: 171.6 against
+ * 197.8). */
+constexpr uint32_t kFixedRounds = 3;
+
 /* The sweep over the bricks some view keeps: list holds them in ascending order
  * (l3d_launch_tsdf_brick_list), prefix[b] is the number of kept bricks below brick b, so the
- * kept bricks of [b_begin, b_end) are list[prefix[b_begin] .. prefix[b_end]).  A
- * warp's pass takes 32 quads of a brick.  Every warp starts with a share of passes by its number and takes
- * the next ones from *next (zeroed before the launch, see there) until none is left: bricks cost as much
- * as views keep them, and a fixed share for each warp leaves warps idle at the end (24 views into 512^3: 322
+ * kept bricks of [b_begin, b_end) are list[prefix[b_begin] .. prefix[b_end]).  A warp's pass takes 32
+ * quads of a brick.  Every warp starts with a share of passes by its number and, beyond kFixedRounds,
+ * takes the next ones from *next (zeroed before the launch) until none is left: bricks cost as much as
+ * views keep them, and a fixed share for each warp leaves warps idle at the end (24 views into 512^3: 322
  * us, handed out 270 us).  A share is at most a brick, for few atomics, and an eighth of what there is for
  * each warp, at least a pass: whole bricks left most of the chip waiting for warps that walked their 4
  * or 16 passes alone where few bricks are kept (host call, 24 views of 320x240: 101^3 278 -> 147 us, 256^3
@@ -855,6 +861,7 @@ __global__ void __launch_bounds__(256, 4) k_integrate_many_list(const L3dTsdfGri
     const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t share = min(max(passes / (warps * 8u), 1u), PASSES);
+    const bool fixed = passes <= warps * kFixedRounds;
     uint32_t at = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     for (;;) {
         const uint32_t begin = at * share, end = min(begin + share, passes);
@@ -864,9 +871,12 @@ __global__ void __launch_bounds__(256, 4) k_integrate_many_list(const L3dTsdfGri
                                       b * PER + (i % PASSES) * 32u + lane);
             __syncwarp();
         }
-        if (end >= passes || warps * share >= passes) return;
-        if (lane == 0) at = atomicAdd(next, 1u);
-        at = warps + __shfl_sync(0xffffffffu, at, 0);
+        if (fixed) {
+            at += warps;
+        } else {
+            if (lane == 0) at = atomicAdd(next, 1u);
+            at = warps + __shfl_sync(0xffffffffu, at, 0);
+        }
         if (at * share >= passes) return;
     }
 }
@@ -1396,8 +1406,8 @@ cudaError_t l3d_launch_tsdf_many_list(const L3dTsdfGrid& g, const L3dTsdfView* v
     if (smem > 48 * 1024 || !ordinary)
         return l3d_launch_tsdf_many_range(g, views_dev, n_views, coords, mask, depth_ptrs_dev, priors,
                                           normals, tsdf, weight, q8, q_begin, q_end, stream);
-    /* where even all bricks kept are a pass or less for each warp, none of them asks */
-    if ((b1 - b0) * (per / 32) > (long long)blocks * 8) {
+    /* where even all bricks kept are no more than the fixed rounds, no warp asks */
+    if ((b1 - b0) * (per / 32) > (long long)blocks * 8 * kFixedRounds) {
         const cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
         if (e != cudaSuccess) return e;
     }

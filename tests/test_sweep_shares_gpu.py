@@ -1,6 +1,7 @@
-"""The sweep's hand-out of passes to warps (k_integrate_many_list), where its share changes: as many passes as
-warps or fewer, one pass a share, two or three (of 4 and of 16 a brick), a whole brick; at once and in the
-slabs of a read-back.  Every brick is kept, and the volume equals the views integrated one by one."""
+"""The sweep's hand-out of passes to warps (k_integrate_many_list), where its rule changes: as many passes as
+warps or fewer, a few rounds by the warps' numbers, then asking for one pass a share, two or three (of 4
+and 2 and 13 of 16 a brick), a whole brick; at once and in the slabs of a read-back.  Every brick is kept,
+and the volume equals the views integrated one by one."""
 import numpy as np
 import pytest
 
@@ -13,8 +14,8 @@ pytestmark = pytest.mark.gpu
 
 
 # 4736 warps (148 SMs); 4 passes a brick where the rows are multiples of four, else 16
-@pytest.mark.parametrize("dims", [(64, 64, 64), (72, 64, 64), (104, 104, 104), (216, 216, 216), (248, 248, 248),
-                                  (288, 288, 280), (61, 37, 55), (135, 133, 131), (253, 251, 249)])
+@pytest.mark.parametrize("dims", [(64, 64, 64), (72, 64, 64), (104, 104, 104), (128, 128, 128), (216, 216, 216), (248, 248, 248),
+                                  (288, 288, 280), (61, 37, 55), (66, 66, 66), (101, 99, 101), (135, 133, 131), (253, 251, 249)])
 @pytest.mark.parametrize("q8", [False, True])
 def test_sweep_equals_views_one_by_one(dims, q8):
     voxel = 2.0 / max(dims)
