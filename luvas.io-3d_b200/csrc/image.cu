@@ -60,15 +60,16 @@ enum BlockKind { BLOCK_LUMA, BLOCK_RGB, BLOCK_GRAY };
  * integer (2^-40 away at least, or equal), and the integer division gives the same byte.
  * 2^shift lanes share a block's columns: a lane alone walks a 32 x 32 block in 1024 steps (1280 x 960 to
  * 40 x 30: 141 us, with 32 lanes 19; to a 160 x 120 thumbnail 11.4 -> 7.2 us, with FP64 sums and
- * divisions before).  WIDE: sums beyond 32 bits. */
-template <int KIND, bool WORDS, bool WIDE>
+ * divisions before).  ALONE: one lane per block, its loads at constant steps (8000 x 6000 gray to 1000 x 750:
+ * 16.4 us, 22.6 with the step in a register; not for RGB, whose 2 x 2 blocks it slows).  WIDE: sums beyond 32 bits. */
+template <int KIND, bool WORDS, bool WIDE, bool ALONE>
 __global__ void __launch_bounds__(256) k_blocks(const uint8_t* __restrict__ src, int W, int H, int tw, int th, double sx,
                                                 double sy, int shift, uint8_t* __restrict__ out) {
     using sum_t = typename std::conditional<WIDE, unsigned long long, uint32_t>::type;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long pixels = (long long)tw * th;
-    const int lanes = 1 << shift, lane = (int)t & (lanes - 1);
-    const long long o = t >> shift;
+    const int lanes = ALONE ? 1 : 1 << shift, lane = ALONE ? 0 : (int)t & (lanes - 1);
+    const long long o = ALONE ? t : t >> shift;
     const int i = (int)(o < pixels ? o : pixels - 1); /* every lane takes part in the sums */
     const int y = i / tw, x = i - y * tw;
     int x0, x1, y0, y1;
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(256) k_blocks(const uint8_t* __restrict__ src,
     sum_t a = 0, b = 0, c = 0;
     for (int yy = y0; yy < y1; yy++) {
         const long long row = (long long)yy * W;
-#pragma unroll 2
+#pragma unroll (KIND == BLOCK_GRAY && ALONE ? 4 : 2)
         for (int xx = x0 + lane; xx < x1; xx += lanes) {
             if (KIND == BLOCK_GRAY) {
                 a += src[row + xx];
@@ -228,23 +229,30 @@ inline unsigned blocks_for(long long n) { return (unsigned)((n + 255) / 256); }
 
 inline bool on_words(const uint8_t* p) { return ((size_t)p & 3) == 0; }
 
+/* Threads that fill the chip for gray bytes: a lane's load is one byte there, so lanes that are not needed to
+ * fill it only split rows that one thread reads from the same sectors (4000 x 3000 to 500 x 375: eight lanes
+ * 19.2 us, one 6.2; to 200 x 150: sixteen 20.5, four 11.3; 2^17 threads: 13.9). */
+constexpr long long kGrayThreads = 1 << 16;
+
 template <int KIND>
 cudaError_t launch_blocks(const uint8_t* src, int W, int H, int tw, int th, uint8_t* out, cudaStream_t s) {
     const double sx = (double)W / tw, sy = (double)H / th;
     /* lanes per block: up to a warp, none without a pixel; blocks of less than eight columns are one
      * lane's (1280 x 960 to RGB means of 4 x 4: one lane 5.7 us, four 7.5; 8 x 8: 9.7, eight lanes 7.2) */
     int shift = 0;
+    const long long pixels = (long long)tw * th;
     if (sx >= 8.0)
-        while (shift < 5 && (2 << shift) <= sx) shift++;
-    const long long threads = ((long long)tw * th) << shift;
+        while (shift < 5 && (2 << shift) <= sx && (KIND != BLOCK_GRAY || pixels << shift < kGrayThreads)) shift++;
+    const long long threads = pixels << shift;
     const unsigned grid = (unsigned)((threads + 255) / 256);
     const bool words = KIND != BLOCK_GRAY && on_words(src);
     /* the largest block's sums (and twice its count times 256) fit 32 bits below 2^15 pixels */
     const bool wide = (sx + 1.0) * (sy + 1.0) >= 32768.0;
-    if (wide && words) k_blocks<KIND, KIND != BLOCK_GRAY, true><<<grid, 256, 0, s>>>(src, W, H, tw, th, sx, sy, shift, out);
-    else if (wide) k_blocks<KIND, false, true><<<grid, 256, 0, s>>>(src, W, H, tw, th, sx, sy, shift, out);
-    else if (words) k_blocks<KIND, KIND != BLOCK_GRAY, false><<<grid, 256, 0, s>>>(src, W, H, tw, th, sx, sy, shift, out);
-    else k_blocks<KIND, false, false><<<grid, 256, 0, s>>>(src, W, H, tw, th, sx, sy, shift, out);
+    constexpr bool RGBA = KIND != BLOCK_GRAY, ONE = KIND != BLOCK_RGB;
+    auto* kernel = wide ? (words ? k_blocks<KIND, RGBA, true, false> : k_blocks<KIND, false, true, false>)
+                   : shift ? (words ? k_blocks<KIND, RGBA, false, false> : k_blocks<KIND, false, false, false>)
+                           : (words ? k_blocks<KIND, RGBA, false, ONE> : k_blocks<KIND, false, false, ONE>);
+    kernel<<<grid, 256, 0, s>>>(src, W, H, tw, th, sx, sy, shift, out);
     return cudaGetLastError();
 }
 
