@@ -3047,7 +3047,7 @@ int area_resample(const uint8_t* src, bool rgba, int w, int h, int tw, int th, u
     if (rc) return rc;
     float* temp = nullptr;
     cudaError_t e = cudaSuccess;
-    if (l3d_area_needs_temp(c.cols, c.rows)) e = pool_alloc((void**)&temp, (size_t)tw * h * 4, s);
+    if (l3d_area_needs_temp(c.cols, c.rows, rgba, tw, th)) e = pool_alloc((void**)&temp, (size_t)tw * h * 4, s);
     if (e == cudaSuccess) e = l3d_launch_area(src, rgba, w, h, tw, th, c.cols, c.rows, temp, out, s);
     if (temp) cudaFreeAsync(temp, s);
     if (temporary) cudaFreeAsync(c.block, s);

@@ -154,8 +154,12 @@ __global__ void k_area_cols(const float* __restrict__ temp, int tw, int th, cons
  * launch and the intermediate's allocation and trip while footprints are at most AREA_TAPS each way
  * (1280 x 960 to 600 x 450: 12.8 us in two passes, 9.8 in one, back to back 16.0 and 8.4; 7 taps: 10.4 and
  * 9.7).  Larger footprints, whose targets are small images, keep the two passes: a thread walks the whole
- * footprint alone (9 taps: 13.3 and 14.0; 22 taps: 21 and 54).  SMALL: at most four taps. */
+ * footprint alone (9 taps: 13.3 and 14.0; 22 taps: 21 and 54).  So do large targets, where the row sums made
+ * twice cost more than the launch: from 1.5 million pixels of gray bytes (1280 x 960 to 1440 x 1080: 21.9 us in
+ * one pass, 20.5 in two; 4000 x 3000 to 4500 x 3375: 179 and 135) and 2 million of RGBA, whose row sums also
+ * take the luma twice (1600 x 1200: 24.7 either way; 4500 x 3375: 164 and 150).  SMALL: at most four taps. */
 constexpr int AREA_TAPS = 8;
+constexpr long long AREA_GRAY = 1500000, AREA_RGBA = 2000000;
 template <bool RGBA, bool WORDS, bool SMALL>
 __global__ void __launch_bounds__(256) k_area(const uint8_t* __restrict__ src, int W, int tw, int th,
                                               const L3dAreaCover cols, const L3dAreaCover rows,
@@ -278,8 +282,8 @@ cudaError_t l3d_launch_gray_blocks(const uint8_t* rgba, int W, int H, int tw, in
                                    cudaStream_t s) {
     return launch_blocks<BLOCK_LUMA>(rgba, W, H, tw, th, out, s);
 }
-bool l3d_area_needs_temp(const L3dAreaCover& cols, const L3dAreaCover& rows) {
-    return cols.kmax > AREA_TAPS || rows.kmax > AREA_TAPS;
+bool l3d_area_needs_temp(const L3dAreaCover& cols, const L3dAreaCover& rows, bool rgba, int tw, int th) {
+    return cols.kmax > AREA_TAPS || rows.kmax > AREA_TAPS || (long long)tw * th > (rgba ? AREA_RGBA : AREA_GRAY);
 }
 cudaError_t l3d_launch_area(const uint8_t* src, bool rgba, int W, int H, int tw, int th,
                             const L3dAreaCover& cols, const L3dAreaCover& rows, float* temp,

@@ -469,7 +469,7 @@ cudaError_t l3d_launch_gray_blocks(const uint8_t* rgba, int W, int H, int tw, in
                                    cudaStream_t s);
 /* rgba: an RGBA source (its f32 luma), else u8 gray; temp: tw x H floats where l3d_area_needs_temp, else
  * NULL */
-bool l3d_area_needs_temp(const L3dAreaCover& cols, const L3dAreaCover& rows);
+bool l3d_area_needs_temp(const L3dAreaCover& cols, const L3dAreaCover& rows, bool rgba, int tw, int th);
 cudaError_t l3d_launch_area(const uint8_t* src, bool rgba, int W, int H, int tw, int th,
                             const L3dAreaCover& cols, const L3dAreaCover& rows, float* temp,
                             uint8_t* out, cudaStream_t s);
