@@ -720,7 +720,7 @@ int fast_batch(l3d_stereo* s, int n, const int32_t* refs, const l3d_solve_opts* 
     int rc = fast_capacity(s, n);
     if (rc) return rc;
     L3D_CUDA(cudaEventSynchronize(s->staged), "staging wait");
-    int tiles = 0;
+    int tiles = 0, sources = 0;
     for (int i = 0; i < n; i++) {
         long long off = per_view_offsets ? s->offv[refs[i]] : 0;
         L3dFastView v = fast_view(s, refs[i], &opts[i], off);
@@ -730,6 +730,7 @@ int fast_batch(l3d_stereo* s, int n, const int32_t* refs, const l3d_solve_opts* 
         s->fviews_host[i] = v;
         s->tile_start_host[i] = tiles;
         tiles += v.tiles_x * ((v.H + 7) / 8);
+        sources += v.n;
         if (v.has_prior) {
             L3D_CUDA(cudaMemcpyAsync(prior + off, opts[i].prior, (size_t)v.W * v.H * sizeof(float),
                                      cudaMemcpyHostToDevice, s->stream), "prior upload");
@@ -746,6 +747,7 @@ int fast_batch(l3d_stereo* s, int n, const int32_t* refs, const l3d_solve_opts* 
     d.tile_start = s->tile_start_dev;
     d.n_views = n;
     d.total_tiles = tiles;
+    d.sources = (sources + n - 1) / n;
     d.images = s->images;
     d.pairs = s->pairs;
     d.storage = s->opts.storage;

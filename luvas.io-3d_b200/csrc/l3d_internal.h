@@ -157,6 +157,7 @@ struct L3dFastDev {
     const int* tile_start;     /* n_views + 1 prefix sums of tiles per view */
     int n_views;
     int total_tiles;
+    int sources;               /* per view, the mean rounded up */
     const void* images;        /* linear storage (BF16 sampling path) */
     const uint32_t* pairs;     /* pair image (half2 of a texel and its right neighbour) or NULL */
     int storage;               /* L3D_DTYPE_F32/F16 (texture path) or BF16 (loads) */

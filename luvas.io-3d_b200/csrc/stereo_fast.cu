@@ -49,23 +49,29 @@ constexpr int TX = 16;   /* colour columns per tile */
 constexpr int TY = 8;    /* rows per tile */
 constexpr int S = 36;    /* 6 x 6 window, offsets -5, -3, ..., 5 */
 /* How the propagate step is laid out for one evaluator: resident blocks per SM of the kernel with a
- * thread per pixel and of the one with eight lanes per pixel (l3d_lanes.cuh), and the largest launch,
- * in 128-pixel tiles of one colour, that takes the lanes. */
+ * thread per pixel and of the one with eight lanes per pixel (l3d_lanes.cuh), and the largest launches,
+ * in 128-pixel tiles of one colour, that take the lanes: with one source per view, two, and more.  What the
+ * lanes do eight times over (random numbers, rays, the windows' sums) is done once per candidate however
+ * many sources share it, so with few of them the thread per pixel wins earlier. */
 struct Layout {
-    int blocks, lane_blocks, lane_tiles;
+    int blocks, lane_blocks, lane_tiles[3];
 };
 /* Measured at 640x480, 8 sources, 3 iterations (ms, thread / lanes), 300, 675, 1200, 2400, 4800
  * tiles.  Filtered samples keep the texture pipe busy either way; the lanes win while the thread
  * kernel's last wave is a large part of it: 1.25 / 0.97, 2.36 / 2.04, 3.99 / 3.69, 7.69 / 7.57,
  * 15.7 / 15.8. */
-constexpr Layout kFilter = {5, 5, 3000};
+constexpr Layout kFilter = {5, 5, {450, 1000, 3000}};
+/* (FP16, 3 iterations, thread / lanes, one source: 300 tiles 0.37 / 0.37, 675 0.59 / 0.70, 1200 0.92 / 1.17;
+ * two: 675 1.07 / 0.96, 1200 1.58 / 1.62, 2400 2.82 / 3.08; three: 2400 4.14 / 4.02.)  BF16 loads keep the
+ * LSU busy instead: four sources 300 tiles 2.47 / 1.76, 675 3.84 / 3.79, 2400 13.4 / 13.6, 4800 25.4 / 27.5. */
+constexpr Layout kLinear = {5, 5, {450, 1000, 1000}};
 /* Gathers are bound by latency and issue; a quarter of the lanes idle in the lanes' second round:
  * 1.81 / 1.54, 4.00 / 3.24, 5.68 / 5.75. */
-constexpr Layout kGather = {4, 5, 1000};
+constexpr Layout kGather = {4, 5, {1000, 1000, 1000}};
 /* The exact evaluator likewise: 2.13 / 1.72, 4.41 / 3.77, 6.47 / 6.81.  With four blocks the compiler
  * has the registers to keep a row's gathers in flight, which is worth more than warps (four views,
  * 5 iterations, thread per pixel: 3 blocks 35.6 ms, 4 35.9 ms, 5 38.9 ms). */
-constexpr Layout kExact = {4, 4, 1000};
+constexpr Layout kExact = {4, 4, {1000, 1000, 1000}};
 
 __device__ __forceinline__ float dot3f(float3 a, float3 b) {
     return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x));
@@ -409,7 +415,7 @@ struct Scene {
 template <bool TEX, int TEXROWS = 6, bool COMP = false, bool GATHER = false>
 struct Fast : Scene {
     template <int STRIDE> using Pix = FPix<STRIDE>;
-    static constexpr Layout kLayout = GATHER ? kGather : kFilter;
+    static constexpr Layout kLayout = GATHER ? kGather : TEX ? kFilter : kLinear;
     /* window rows unrolled together: filtered samples want all their fetches in flight, a gather's
      * row of blends is long enough that more than two overflow the instruction cache (four views of
      * 640x480, 8 sources, 5 iterations: 33.6 ms, all six rows 34.6; filtered 23.9 and 23.6) */
@@ -965,7 +971,8 @@ cudaError_t launch_eval(int kernel, const L3dFastDev& d, int iteration, int phas
         k_fast_init<E><<<d.total_tiles, 128, 0, st>>>(d);
     } else {
         float step = ldexpf(1.0f, -iteration);
-        if (d.total_tiles <= E::kLayout.lane_tiles)
+        const int sources = d.sources < 1 ? 1 : d.sources > 3 ? 3 : d.sources;
+        if (d.total_tiles <= E::kLayout.lane_tiles[sources - 1])
             k_fast_propagate_lanes<E><<<d.total_tiles * PARTS, 128, 0, st>>>(d, iteration, phase, step);
         else
             k_fast_propagate<E><<<d.total_tiles, 128, 0, st>>>(d, iteration, phase, step);
